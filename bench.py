@@ -827,22 +827,16 @@ def run_fdtd2d(args):
         e1.record()
         torch.cuda.synchronize(dev)
         s_solve = e0.elapsed_time(e1) / 1e3 / reps
-        # gradient-free solves that fit one thread-block cluster run as one
-        # launch per solve; the others launch the step kernel once per step
-        batch = next((v for v in solver.__dict__.get("_cluster_cache", {}).values()
-                      if v is not None), None)
-        cluster = batch is not None
-        kernel = "k_fdtd2d_step"
-        if cluster:
-            from diffnano_b200 import _lib
-
-            db = batch._cluster[0] & _lib.DN_CLUSTER_DOUBLE_BUFFERED
-            kernel = "k_batch2d_cluster_db" if db else "k_batch2d_cluster"
+        # grids that fit on the chip take all steps in one launch (and one for the
+        # monitor's DFT); the others launch the step kernel once per step
+        eng = next(iter(solver.__dict__["_engine_cache"].values()))
+        resident = eng._workspace()[1] > 0
+        kernel = "k_resident2d" if resident else "k_fdtd2d_step"
         out[key] = {"grid": side, "steps": T, "s_per_solve": s_solve,
                     "gcells": side * side * T / s_solve / 1e9,
                     "gbs": 28 * side * side * T / s_solve / 1e9,
                     "kernel": kernel, "warmup_solves": n_warm, "timed_solves": reps,
-                    "launches_per_solve": 1 if cluster else T}
+                    "launches_per_solve": 2 if resident else T}
         if not args.no_fp64_check:
             s64 = FDTDSolver2D(grid_shape=(side, side), dl=st.dl, wavelength_nm=st.center_nm,
                                pml_layers=st.pml, n_steps=T, courant=st.courant, device=dev,

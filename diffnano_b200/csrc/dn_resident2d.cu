@@ -1,0 +1,305 @@
+// Resident 2-D runs (dn_resident2d.cuh): the choice of the work split, the
+// workspace and the entry points.
+#include <algorithm>
+
+#include "dn_resident2d.cuh"
+#include "dn_strip.cuh"
+
+namespace dn {
+namespace res {
+namespace {
+
+// ---- monitors ------------------------------------------------------------------
+// The march only stores each step's values of a monitor's cells (samples, the
+// grid's type); their running DFT is added to the monitor's FP64 sums by a
+// kernel of its own after the run, which keeps FP64 arithmetic and its
+// registers out of the step every other warp waits for.
+//
+// sums[f][cell] += sum_t sample[t][cell] phase[t][f]: a block owns 32 cells, its
+// warps take every DFT_WARPS-th step, and the partial sums are added in warp
+// order (deterministic).
+constexpr int DFT_WARPS = 16;
+constexpr int DFT_FREQS = 4;  // frequencies per pass
+template <typename T>
+__global__ void __launch_bounds__(DFT_WARPS * 32)
+    k_sample_dft(const T* __restrict__ smp, long long step_stride, int nsteps, long long ncell,
+                 const double* __restrict__ phase, int nf, double* __restrict__ acc,
+                 const int* status) {
+  if (status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;
+  __shared__ double2 part[DFT_WARPS][DFT_FREQS][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const long long cell = (long long)blockIdx.x * 32 + lane;
+  const bool ok = cell < ncell;
+  for (int f0 = 0; f0 < nf; f0 += DFT_FREQS) {
+    double2 s[DFT_FREQS];
+#pragma unroll
+    for (int f = 0; f < DFT_FREQS; ++f) s[f] = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int t = w; t < nsteps; t += DFT_WARPS) {
+      const double x = ok ? static_cast<double>(smp[t * step_stride + cell]) : 0.0;
+      const double* ph = phase + ((long long)t * nf + f0) * 2;
+#pragma unroll
+      for (int f = 0; f < DFT_FREQS; ++f)
+        if (f0 + f < nf) {
+          s[f].x = fma(x, __ldg(ph + 2 * f), s[f].x);
+          s[f].y = fma(x, __ldg(ph + 2 * f + 1), s[f].y);
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < DFT_FREQS; ++f) part[w][f][lane] = s[f];
+    __syncthreads();
+    for (int e = threadIdx.x; e < DFT_FREQS * 32; e += blockDim.x) {
+      const int f = e / 32, l = e % 32;
+      const long long c = (long long)blockIdx.x * 32 + l;
+      if (f0 + f < nf && c < ncell) {
+        double2 u = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int v = 0; v < DFT_WARPS; ++v) {
+          u.x += part[v][f][l].x;
+          u.y += part[v][f][l].y;
+        }
+        double* a = acc + ((long long)(f0 + f) * ncell + c) * 2;
+        a[0] += u.x;
+        a[1] += u.y;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The work split of a grid, or none (R = 0) when it does not fit on the chip.
+//
+// A step costs what the busiest warp's block costs (rows per warp) plus the
+// trip of a row to the next band.  Measured on B200, FP32 TM, us per step: one
+// cluster (at most 16 bands) 0.41 (R = 1, 8 warps), 0.55 (R = 1, 16 warps),
+// 0.45 / 0.48 / 0.76 (R = 2; 4 / 8 / 16 warps); bands over the whole chip 0.7 -
+// 0.95 (R = 1), 1.0 - 1.2 (R = 2), 1.6 - 2.0 (R = 3), 1.9 - 2.2 (R = 4), where
+// one launch per step takes 6.2 (256 x 256) to 8.3 (1024 x 1024).  So: a cluster
+// where 16 bands hold the grid, else the fewest rows per warp for which one
+// band per SM does.
+Split choose_split(int H, int W, int elem, int nsm) {
+  Split S{};
+  const int cols = 32 * 16 / elem;
+  const int strips = (W + cols - 1) / cols;
+  auto fits = [&](int R, int bands) {
+    const int groups = std::max(1, (H + bands * R - 1) / (bands * R));
+    if (strips * groups > MAX_WARPS) return false;
+    S = Split{R, strips, groups, (H + groups * R - 1) / (groups * R), 0};
+    return true;
+  };
+  if (fits(1, 16) && S.strips * S.groups <= 8) return S.cluster = 1, S;
+  if (fits(2, 16)) return S.cluster = 1, S;
+  for (int R = 1; R <= 4; ++R)
+    if (fits(R, nsm)) return S;
+  return Split{};
+}
+
+constexpr long long SAMPLE_BYTES = 64LL << 20;  // most workspace for samples
+constexpr int MIN_STEPS = 8;  // shorter runs (or pieces between DFTs) go launch by launch
+
+// everything a run needs, or ok = false for the launch-by-launch path
+struct Plan2d {
+  bool ok;
+  Split S;
+  long long mail_bytes;    // the two mailboxes of every band
+  long long sample_bytes;  // one step's samples of all monitors
+  int piece;               // steps per launch (whole run, or what the samples allow)
+};
+
+Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mons, int n_mon,
+                   int nsteps) {
+  Plan2d P{};
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return P;
+  const int elem = g->dtype == DN_F32 ? 4 : 8;
+  const int first = g->pol == DN_TM ? DN_EZ : DN_HZ;
+  if (nsteps < MIN_STEPS || (g->pitch_y * elem) % 16 != 0) return P;
+  if (src && src->component != DN_NONE && src->component != first) return P;
+  // the TE update of these equations grows without bound (FP32 overflows within
+  // ~130 steps): FP32 TE runs are short, and stay launch by launch
+  if (g->pol == DN_TE && g->dtype == DN_F32) return P;
+  P.S = choose_split(g->H, g->W, elem, nsm);
+  if (P.S.R == 0) return P;
+  P.mail_bytes = P.S.cluster ? 0 : (long long)P.S.bands * 4 * P.S.strips * ROW_WORDS * 8;
+  P.piece = nsteps;
+  for (int m = 0; m < n_mon; ++m)
+    P.sample_bytes += (to_dev(mons[m].box).cells() * elem + 15) / 16 * 16;
+  if (P.sample_bytes * nsteps > SAMPLE_BYTES) {
+    P.piece = (int)(SAMPLE_BYTES / P.sample_bytes);
+    if (P.piece < 4 * MIN_STEPS) return P;
+  }
+  P.ok = true;
+  return P;
+}
+
+long long workspace_of(const Plan2d& P) {
+  return P.ok ? P.mail_bytes + P.sample_bytes * P.piece : 0;
+}
+
+template <typename T>
+int run2d_resident(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
+                   const dn_cpml* cpml, const StepParams<T>& p, const dn_probe* probe,
+                   const dn_curl_record* crec, int t0, int nsteps, int* status, cudaStream_t s,
+                   const Plan2d& P, unsigned char* ws) {
+  const bool tm = g->pol == DN_TM;
+  const int comp[3] = {tm ? DN_EZ : DN_HZ, tm ? DN_HX : DN_EX, tm ? DN_HY : DN_EY};
+  Job<T> J{};
+  J.H = g->H;
+  J.W = g->W;
+  J.py = g->pitch_y;
+  J.ce = static_cast<const T*>(ce);
+  for (int a = 0; a < 2; ++a) {
+    J.b[a] = cpml->b[1 + a];
+    J.c[a] = cpml->c[1 + a];
+    J.src_lo[a] = p.src.box.lo[1 + a];
+    J.src_hi[a] = p.src.box.hi[1 + a];
+  }
+  J.dt = g->dt;
+  J.dl = g->dl;
+  J.src = p.src.comp >= 0;
+  J.wave = p.src.wave;
+  constexpr int VEC = 16 / (int)sizeof(T);
+  for (int n = 0; n < nsteps; n += P.piece) {
+    const int k = std::min(P.piece, nsteps - n);
+    J.t0 = t0 + n;
+    J.nsteps = k;
+    for (int c = 0; c < 3; ++c) {
+      void* const to = nsteps % 2 ? fb[comp[c]] : fa[comp[c]];
+      J.in[c] = static_cast<const T*>(n == 0 ? fa[comp[c]] : to);
+      J.out[c] = static_cast<T*>(to);
+    }
+    if (crec) {
+      J.curl_stride = crec->step_stride;
+      for (int c = 0; c < (tm ? 1 : 2); ++c)
+        J.curl[c] = static_cast<T*>(crec->curl[tm ? 2 : c]) +
+                    (long long)(t0 + n - crec->t0) * crec->step_stride;
+    }
+    SampleSet<T> set{};
+    unsigned char* at = ws + P.mail_bytes;
+    auto add = [&](int c, const BoxDev& b, T* buf, long long stride) {
+      Samples<T>& q = set.s[set.n++];
+      for (int a = 0; a < 2; ++a) {
+        q.lo[a] = b.lo[1 + a];
+        q.hi[a] = b.hi[1 + a];
+      }
+      q.comp = c == comp[0] ? 0 : c == comp[1] ? 1 : 2;
+      q.vec = q.lo[1] % VEC == 0 && (q.hi[1] - q.lo[1]) % VEC == 0;
+      q.buf = buf;
+      q.step_stride = stride;
+    };
+    for (int m = 0; m < p.n_mon; ++m) {
+      const long long stride = (p.mon[m].ncell * (long long)sizeof(T) + 15) / 16 * 16 / sizeof(T);
+      add(p.mon[m].comp, p.mon[m].box, reinterpret_cast<T*>(at), stride);
+      at += stride * sizeof(T) * k;
+    }
+    if (p.probe.comp >= 0) {
+      BoxDev b{};
+      for (int a = 0; a < 3; ++a) b.lo[a] = p.probe.pos[a], b.hi[a] = p.probe.pos[a] + 1;
+      add(p.probe.comp, b, p.probe.out + t0 + n, 1);
+      set.s[set.n - 1].vec = 0;
+    }
+    if (P.mail_bytes) DN_CUDA_CHECK(cudaMemsetAsync(ws, 0, P.mail_bytes, s));
+    uint64_t* const mail = reinterpret_cast<uint64_t*>(ws);
+    int rc = DN_EINVAL;
+    if (tm)
+      rc = run_resident<T, DN_TM>(J, set, P.S, mail, status, s);
+    else if constexpr (sizeof(T) == 8)
+      rc = run_resident<T, DN_TE>(J, set, P.S, mail, status, s);
+    if (rc != DN_OK) return rc;
+    for (int m = 0; m < p.n_mon; ++m) {
+      const MonDev& M = p.mon[m];
+      k_sample_dft<T><<<(unsigned)((M.ncell + 31) / 32), DFT_WARPS * 32, 0, s>>>(
+          set.s[m].buf, set.s[m].step_stride, k, M.ncell,
+          M.phase + (long long)(t0 + n) * M.nf * 2, M.nf, M.acc, status);
+    }
+    DN_CUDA_CHECK(cudaGetLastError());
+  }
+  return DN_OK;
+}
+
+// 16-byte rows: every array the polarisation uses, and the curl slots
+template <typename T>
+bool rows_ok(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
+             const dn_curl_record* rec) {
+  const int comps[2][3] = {{DN_EZ, DN_HX, DN_HY}, {DN_HZ, DN_EX, DN_EY}};
+  const int tm = g->pol == DN_TM;
+  if (!aligned16(ce)) return false;
+  for (int c : comps[tm ? 0 : 1])
+    if (!aligned16(fa[c]) || !aligned16(fb[c])) return false;
+  if (rec) {
+    if ((rec->step_stride * (long long)sizeof(T)) % 16 != 0) return false;
+    if (tm ? !aligned16(rec->curl[2]) : !aligned16(rec->curl[0]) || !aligned16(rec->curl[1]))
+      return false;
+  }
+  return true;
+}
+
+template <typename T>
+int run_ws(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
+           const dn_cpml* cpml, const dn_source* src, const dn_monitor* mons, int32_t n_mon,
+           const dn_probe* probe, const dn_curl_record* rec, int32_t t0, int32_t nsteps,
+           int32_t* status, cudaStream_t s, int32_t* final_in_b, void* ws, int64_t ws_bytes,
+           bool* done) {
+  *done = false;
+  StepParams<T> p;
+  const int rc = build_params<T>(false, g, fa, fb, ce, cpml, src, mons, n_mon, probe, status, &p);
+  if (rc != DN_OK) return rc;
+  if (t0 < 0 || !final_in_b || !steps_ok(src, mons, n_mon, probe, t0, (int64_t)t0 + nsteps))
+    return DN_EINVAL;
+  if (rec) {
+    const bool tm = g->pol == DN_TM;
+    if ((tm && !rec->curl[2]) || (!tm && (!rec->curl[0] || !rec->curl[1]))) return DN_EINVAL;
+    if (rec->step_stride < (int64_t)g->H * g->pitch_y || rec->t0 < 0 || t0 < rec->t0 ||
+        t0 + nsteps > rec->t0 + rec->nslots)
+      return DN_EINVAL;
+  }
+  const Plan2d P = make_plan2d(g, src, mons, n_mon, nsteps);
+  if (!P.ok || workspace_of(P) > ws_bytes || !aligned16(ws) || !rows_ok<T>(g, fa, fb, ce, rec))
+    return DN_OK;
+  *done = true;
+  const int r2 = run2d_resident<T>(g, fa, fb, ce, cpml, p, probe, rec, t0, nsteps, status, s, P,
+                                   static_cast<unsigned char*>(ws));
+  if (r2 == DN_OK) *final_in_b = nsteps % 2;
+  return r2;
+}
+
+}  // namespace
+}  // namespace res
+}  // namespace dn
+
+extern "C" int64_t dn_fdtd2d_workspace_bytes(const dn_grid* g, const dn_source* src,
+                                             const dn_monitor* mons, int32_t n_mon,
+                                             int32_t nsteps) {
+  if (!g || g->H < 1 || g->W < 1 || g->D != 1 || (g->dtype != DN_F32 && g->dtype != DN_F64) ||
+      (g->pol != DN_TM && g->pol != DN_TE) || n_mon < 0 || n_mon > DN_MAX_MONITORS ||
+      (n_mon > 0 && !mons))
+    return -1;
+  for (int m = 0; m < n_mon; ++m)
+    if (!dn::box_ok(mons[m].box, 1, g->H, g->W)) return -1;
+  return dn::res::workspace_of(dn::res::make_plan2d(g, src, mons, n_mon, nsteps));
+}
+
+extern "C" int32_t dn_fdtd2d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],
+                                    const void* ce, const dn_cpml* cpml, const dn_source* src,
+                                    const dn_monitor* mons, int32_t n_mon, const dn_probe* probe,
+                                    const dn_curl_record* rec, int32_t t0, int32_t nsteps,
+                                    int32_t* status, void* stream, int32_t* final_in_b, void* ws,
+                                    int64_t ws_bytes) {
+  if (!g) return DN_EINVAL;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (nsteps >= dn::res::MIN_STEPS && (ws || ws_bytes == 0)) {
+    bool done = false;
+    int rc = DN_OK;
+    if (g->dtype == DN_F32)
+      rc = dn::res::run_ws<float>(g, fa, fb, ce, cpml, src, mons, n_mon, probe, rec, t0, nsteps,
+                                  status, s, final_in_b, ws, ws_bytes, &done);
+    else if (g->dtype == DN_F64)
+      rc = dn::res::run_ws<double>(g, fa, fb, ce, cpml, src, mons, n_mon, probe, rec, t0, nsteps,
+                                   status, s, final_in_b, ws, ws_bytes, &done);
+    if (rc != DN_OK || done) return rc;
+  }
+  return dn_fdtd2d_run(g, fa, fb, ce, cpml, src, mons, n_mon, probe, rec, t0, nsteps, status,
+                       stream, final_in_b);
+}

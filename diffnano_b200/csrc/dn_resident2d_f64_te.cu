@@ -1,0 +1,4 @@
+#include "dn_resident2d_fwd.cuh"
+
+template int dn::res::run_resident<double, DN_TE>(const Job<double>&, const SampleSet<double>&, const Split&,
+                                              uint64_t*, int*, cudaStream_t);

@@ -163,6 +163,7 @@ class Engine:
             self.probe.n_t = self.probe_out.numel()
 
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
+        self._ws = None  # 2-D: workspace of the resident runs, made by the first run
 
     # ------------------------------------------------------------------
     def set_eps(self, eps: torch.Tensor) -> None:
@@ -208,20 +209,30 @@ class Engine:
         L = _lib.lib()
         fa, fb = (self.B, self.A) if self.cur_b else (self.A, self.B)
         out = ctypes.c_int32(0)
-        fn_name = "dn_fdtd3d_run" if self.is3d else "dn_fdtd2d_run"
+        fn_name = "dn_fdtd3d_run" if self.is3d else "dn_fdtd2d_run_ws"
         no_probe = _lib.DnProbe(component=_lib.DN_NONE)
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device).cuda_stream
+            ws = () if self.is3d else self._workspace()
             rc = getattr(L, fn_name)(
                 ctypes.byref(self.grid), self._ptrs(fa), self._ptrs(fb), self.ce.data_ptr(),
                 ctypes.byref(self.cpml), ctypes.byref(self.src), self.mon_arr,
                 len(self.monitors) if outputs else 0,
                 ctypes.byref(self.probe if outputs else no_probe),
                 ctypes.byref(record) if record is not None else None, int(t0), int(nsteps),
-                self.status.data_ptr(), ctypes.c_void_p(stream), ctypes.byref(out))
+                self.status.data_ptr(), ctypes.c_void_p(stream), ctypes.byref(out), *ws)
         _lib.check(fn_name, rc)
         if out.value:
             self.cur_b = not self.cur_b
+
+    def _workspace(self):
+        """(pointer, bytes) of the 2-D runs' workspace, enough for the longest run."""
+        if self._ws is None:
+            n = int(_lib.lib().dn_fdtd2d_workspace_bytes(
+                ctypes.byref(self.grid), ctypes.byref(self.src), self.mon_arr,
+                len(self.monitors), self.n_steps))
+            self._ws = torch.empty(max(n, 0), dtype=torch.uint8, device=self.device)
+        return self._ws.data_ptr() if self._ws.numel() else None, self._ws.numel()
 
     # ------------------------------------------------------------------
     # adjoint support

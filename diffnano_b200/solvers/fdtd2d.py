@@ -2,7 +2,8 @@
 
 Same constructor, attributes, ``forward`` and ``time_series`` as the
 reference (``diffnano/solvers/fdtd2d.py:91-524``); every time step runs in the
-``dn_fdtd2d_run`` CUDA kernel (``include/dn_fdtd.h``).  Additions, all
+CUDA kernels behind ``dn_fdtd2d_run_ws`` (``include/dn_fdtd.h``): grids that fit on
+the chip take all steps in one launch, larger ones one launch per step.  Additions, all
 optional keyword arguments: ``backward`` ("auto"/"autograd"/"time_reversal"/
 "checkpoint"), ``dtype`` (torch.float32 default, torch.float64 for
 validation), and DFT ``monitors``.
@@ -13,7 +14,6 @@ from __future__ import annotations
 import json
 import math
 from collections.abc import Sequence
-from types import SimpleNamespace
 
 import torch
 
@@ -117,37 +117,24 @@ class FDTDSolver2D:
         eps = self._prep_eps(geometry)
         mons = monitors if monitors is not None else self.monitors
         probe = src.get("probe", None)
-        fast, eng, specs = None, None, None
-        if probe is None and not (torch.is_grad_enabled() and eps.requires_grad):
-            # the cluster-resident path needs only the parsed monitors, not a
-            # per-step engine (field sets, tables and uploads on every call)
-            H, W = self.grid_shape
-            specs = parse_monitors(mons, (1, H, W), False, self.wavelength_nm,
-                                   self._fields()[0], self._fields())
-            fast = self._cluster_solve(eps, src, specs)
-        if fast is not None:
-            field, dfts = fast
-        else:
-            from diffnano_b200.solvers._adjoint import run_forward
+        from diffnano_b200.solvers._adjoint import run_forward
 
-            needs_grad = torch.is_grad_enabled() and eps.requires_grad
-            eng = self._engine_for(src, mons, probe, reuse=not needs_grad)
-            specs = eng.monitors
-            field, dfts = run_forward(self, eng, eps, self._fields()[0])
+        needs_grad = torch.is_grad_enabled() and eps.requires_grad
+        eng = self._engine_for(src, mons, probe, reuse=not needs_grad)
+        field, dfts = run_forward(self, eng, eps, self._fields()[0])
         out_dev = self._device
         snapshots = []
         if probe is not None:
             snapshots = list(eng.probe_out.to(out_dev, copy=True).unbind(0))
         meta = {"polarization": self.polarization, "n_steps": self.n_steps, "dt": self.dt,
                 "courant": self.courant, "snapshots": snapshots}
-        if specs:
-            meta["monitors"] = monitor_metadata(SimpleNamespace(monitors=specs),
-                                                [to_result_device(d, out_dev) for d in dfts])
+        if eng.monitors:
+            meta["monitors"] = monitor_metadata(eng, [to_result_device(d, out_dev) for d in dfts])
         return SimResult(field=to_result_device(field.unsqueeze(0), out_dev), wavelengths=wl,
                          metadata=meta)
 
     def _engine_for(self, src: dict, mons, probe, reuse: bool) -> Engine:
-        """The per-step engine of a solve.  Gradient-free calls reuse one per
+        """The engine of a solve.  Gradient-free calls reuse one per
         set-up (every run resets its fields and writes eps, and the results
         are copies), which saves the field allocations and table uploads of a
         new engine; calls that autograd differentiates get a fresh one, since
@@ -169,44 +156,6 @@ class FDTDSolver2D:
                 cache.clear()
             eng = cache[key] = self._make_engine(self.n_steps, src, mons, probe)
         return eng
-
-    def _cluster_solve(self, eps, src, specs):
-        """Gradient-free solve with the whole grid in one thread-block cluster
-        (``dn_batch2d_forward_cluster``) when the grid fits and there is at most
-        one monitor (``specs``: the parsed monitors), on the injected field;
-        None otherwise."""
-        if len(specs) > 1:
-            return None
-        comp = _lib.DN_EZ if self.polarization == "TM" else _lib.DN_HZ
-        mon = None
-        if specs:
-            m = specs[0]
-            if m.component != comp:
-                return None
-            mon = {"box": [list(m.box[1]), list(m.box[2])], "wavelengths_nm": list(m.wavelengths)}
-        key = json.dumps([src, mon, str(self.dtype), list(self.grid_shape), self.n_steps,
-                          self.dl, self.wavelength_nm, self.pml_layers, self.courant,
-                          self.polarization, str(self._device)], sort_keys=True, default=str)
-        cache = self.__dict__.setdefault("_cluster_cache", {})
-        if key not in cache:
-            from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D
-
-            spec = BatchInstance(grid_shape=tuple(self.grid_shape), n_steps=self.n_steps,
-                                 dl=self.dl, wavelength_nm=self.wavelength_nm,
-                                 pml_layers=self.pml_layers, courant=self.courant,
-                                 source={k: v for k, v in src.items() if k != "probe"},
-                                 monitor=mon)
-            b = FDTDBatch2D([spec], self.polarization, self.dtype,
-                            compute_device(self._device), tile_rows=16)
-            b._build(False)
-            cache[key] = b if b.uses_cluster(False) else None
-        b = cache[key]
-        if b is None:
-            return None
-        with torch.no_grad():
-            fields, dfts = b.run_forward([eps], grad=False)
-        b.check_status()
-        return fields[0], [d for d in dfts if d is not None]
 
     def time_series(self, eps_r: torch.Tensor, probe: tuple[int, int], source: dict | None = None,
                     n_steps: int | None = None) -> torch.Tensor:

@@ -167,6 +167,24 @@ int32_t dn_fdtd2d_run(const dn_grid* g, void* const fa[6], void* const fb[6], co
                       int32_t t0, int32_t nsteps, int32_t* status, void* stream,
                       int32_t* final_in_b);
 
+/* dn_fdtd2d_run with a workspace.  Where the grid fits on the chip, all steps
+ * run in one launch with the fields held in registers (the result is where
+ * *final_in_b says; the other set is left as it was); otherwise, and for short
+ * runs, the steps are launched one by one as by dn_fdtd2d_run.  The workspace
+ * (device memory, 16-byte aligned, contents irrelevant before and after) needs
+ * dn_fdtd2d_workspace_bytes bytes for the longest run it is used with; with a
+ * smaller one (NULL and 0 included) runs that would need more are launched step
+ * by step.  Calls that share a workspace must not overlap in time.
+ * dn_fdtd2d_workspace_bytes: 0 when no workspace would be used, -1 on invalid
+ * input. */
+int64_t dn_fdtd2d_workspace_bytes(const dn_grid* g, const dn_source* src, const dn_monitor* mons,
+                                  int32_t n_mon, int32_t nsteps);
+int32_t dn_fdtd2d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
+                         const dn_cpml* cpml, const dn_source* src, const dn_monitor* mons,
+                         int32_t n_mon, const dn_probe* probe, const dn_curl_record* rec,
+                         int32_t t0, int32_t nsteps, int32_t* status, void* stream,
+                         int32_t* final_in_b, void* ws, int64_t ws_bytes);
+
 /* 3-D analogue (all six components), same ping-pong and status contract.
  * Field bases and ce must be 16-byte aligned, pitches multiples of 16 bytes. */
 int32_t dn_fdtd3d_run(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
