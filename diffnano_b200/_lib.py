@@ -146,6 +146,10 @@ SIGNATURES = {
                                     ctypes.POINTER(DnCpml), ctypes.POINTER(DnCurlRecord),
                                     c_void_p, ctypes.POINTER(DnMonitor), c_int32, c_int32,
                                     c_int32, c_void_p, c_void_p, ctypes.POINTER(c_int32)]),
+    "dn_fdtd2d_adjoint_ws": (c_int32, [ctypes.POINTER(DnGrid), _P6, _P6, c_void_p,
+                                    ctypes.POINTER(DnCpml), ctypes.POINTER(DnCurlRecord),
+                                    c_void_p, ctypes.POINTER(DnMonitor), c_int32, c_int32,
+                                    c_int32, c_void_p, c_void_p, ctypes.POINTER(c_int32), c_void_p, c_int64]),
     "dn_fdtd3d_adjoint": (c_int32, [ctypes.POINTER(DnGrid), _P6, _P6, c_void_p,
                                     ctypes.POINTER(DnCpml), ctypes.POINTER(DnCurlRecord),
                                     c_void_p, ctypes.POINTER(DnMonitor), c_int32, c_int32,

@@ -2,6 +2,7 @@
 // workspace and the entry points.
 #include <algorithm>
 
+#include "dn_adjoint.cuh"
 #include "dn_resident2d.cuh"
 #include "dn_strip.cuh"
 
@@ -76,8 +77,10 @@ __global__ void __launch_bounds__(DFT_WARPS * 32)
 // 0.95 (R = 1), 1.0 - 1.2 (R = 2), 1.6 - 2.0 (R = 3), 1.9 - 2.2 (R = 4), where
 // one launch per step takes 6.2 (256 x 256) to 8.3 (1024 x 1024).  So: a cluster
 // where 16 bands hold the grid, else the fewest rows per warp for which one
-// band per SM does.
-Split choose_split(int H, int W, int elem, int nsm) {
+// band per SM does.  The reverse sweep holds the FP64 gradient too: at most
+// R = 3 (909 k cells in FP32).
+constexpr int R_MAX = 4, R_MAX_ADJ = 3;
+Split choose_split(int H, int W, int elem, int nsm, int r_max) {
   Split S{};
   const int cols = 32 * 16 / elem;
   const int strips = (W + cols - 1) / cols;
@@ -89,7 +92,7 @@ Split choose_split(int H, int W, int elem, int nsm) {
   };
   if (fits(1, 16) && S.strips * S.groups <= 8) return S.cluster = 1, S;
   if (fits(2, 16)) return S.cluster = 1, S;
-  for (int R = 1; R <= 4; ++R)
+  for (int R = 1; R <= r_max; ++R)
     if (fits(R, nsm)) return S;
   return Split{};
 }
@@ -107,7 +110,7 @@ struct Plan2d {
 };
 
 Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mons, int n_mon,
-                   int nsteps) {
+                   int nsteps, bool adjoint) {
   Plan2d P{};
   int dev = 0, nsm = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -119,8 +122,11 @@ Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mon
   if (src && src->component != DN_NONE && src->component != first) return P;
   // the TE update of these equations grows without bound (FP32 overflows within
   // ~130 steps): FP32 TE runs are short, and stay launch by launch
-  if (g->pol == DN_TE && g->dtype == DN_F32) return P;
-  P.S = choose_split(g->H, g->W, elem, nsm);
+  if (g->pol == DN_TE && (adjoint || g->dtype == DN_F32)) return P;
+  // what a monitor adds in the reverse sweep goes to lambda_Ez alone
+  for (int m = 0; adjoint && m < n_mon; ++m)
+    if (mons[m].component != first) return P;
+  P.S = choose_split(g->H, g->W, elem, nsm, adjoint ? R_MAX_ADJ : R_MAX);
   if (P.S.R == 0) return P;
   P.mail_bytes = P.S.cluster ? 0 : (long long)P.S.bands * 4 * P.S.strips * ROW_WORDS * 8;
   P.piece = nsteps;
@@ -255,7 +261,7 @@ int run_ws(const dn_grid* g, void* const fa[6], void* const fb[6], const void* c
         t0 + nsteps > rec->t0 + rec->nslots)
       return DN_EINVAL;
   }
-  const Plan2d P = make_plan2d(g, src, mons, n_mon, nsteps);
+  const Plan2d P = make_plan2d(g, src, mons, n_mon, nsteps, false);
   if (!P.ok || workspace_of(P) > ws_bytes || !aligned16(ws) || !rows_ok<T>(g, fa, fb, ce, rec))
     return DN_OK;
   *done = true;
@@ -265,9 +271,133 @@ int run_ws(const dn_grid* g, void* const fa[6], void* const fb[6], const void* c
   return r2;
 }
 
+// what the monitors add to lambda before reverse steps t, t-1, ..: out[n][cell] =
+// sum_f g[f][cell] . phase[t - n][f]
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_add_table(T* __restrict__ out, long long stride, int nsteps, int t, long long ncell,
+                const double* __restrict__ phase, int nf, const double* __restrict__ g) {
+  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < ncell * nsteps;
+       e += gridDim.x * 256LL) {
+    const long long n = e / ncell, cell = e - n * ncell;
+    const double* ph = phase + (t - n) * nf * 2;
+    double s = 0.0;
+    for (int f = 0; f < nf; ++f) {
+      const double* a = g + ((long long)f * ncell + cell) * 2;
+      s = fma(a[0], __ldg(ph + 2 * f), fma(a[1], __ldg(ph + 2 * f + 1), s));
+    }
+    out[n * stride + cell] = static_cast<T>(s);
+  }
+}
+
+template <typename T>
+int adjoint_ws(const dn_grid* g, void* const la[6], void* const lb[6], const void* ce,
+               const dn_cpml* cpml, const dn_curl_record* curl, double* grad,
+               const dn_monitor* mons, int32_t n_mon, int32_t t_end, int32_t nsteps,
+               int32_t* status, cudaStream_t s, int32_t* final_in_b, unsigned char* ws,
+               int64_t ws_bytes, bool* done) {
+  *done = false;
+  AdjParams<T> p;
+  int rc = build_adj_params<T>(false, g, la, lb, ce, cpml, curl, grad, t_end, nsteps, status, &p);
+  if (rc != DN_OK) return rc;
+  if (!final_in_b || n_mon < 0 || n_mon > DN_MAX_MONITORS || (n_mon > 0 && !mons))
+    return DN_EINVAL;
+  if (!mons_steps_ok(mons, n_mon, (int64_t)t_end - nsteps, t_end)) return DN_EINVAL;
+  for (int m = 0; m < n_mon; ++m)
+    if (!box_ok(mons[m].box, 1, g->H, g->W) || mons[m].n_freq < 1 ||
+        mons[m].n_freq > DN_MAX_FREQS || !mons[m].phase || !mons[m].acc)
+      return DN_EINVAL;
+  const Plan2d P = make_plan2d(g, nullptr, mons, n_mon, nsteps, true);
+  const int comp[3] = {DN_EZ, DN_HX, DN_HY};
+  if (!P.ok || workspace_of(P) > ws_bytes || !aligned16(ws) || !aligned16(ce) ||
+      !aligned16(grad) || !aligned16(curl->curl[2]) ||
+      (curl->step_stride * (long long)sizeof(T)) % 16 != 0)
+    return DN_OK;
+  for (int c : comp)
+    if (!aligned16(la[c]) || !aligned16(lb[c])) return DN_OK;
+  *done = true;
+  AdjJob<T> J{};
+  J.H = g->H;
+  J.W = g->W;
+  J.py = g->pitch_y;
+  J.ce = static_cast<const T*>(ce);
+  for (int a = 0; a < 2; ++a) {
+    J.b[a] = cpml->b[1 + a];
+    J.c[a] = cpml->c[1 + a];
+  }
+  J.dt = g->dt;
+  J.dl = g->dl;
+  J.grad = grad;
+  J.curl_stride = curl->step_stride;
+  constexpr int VEC = 16 / (int)sizeof(T);
+  for (int n = 0; n < nsteps; n += P.piece) {
+    const int k = std::min(P.piece, nsteps - n);
+    const int t = t_end - 1 - n;  // the piece's first reverse step
+    J.nsteps = k;
+    J.curl = static_cast<const T*>(curl->curl[2]) + (long long)(t - curl->t0) * J.curl_stride;
+    for (int c = 0; c < 3; ++c) {
+      void* const to = nsteps % 2 ? lb[comp[c]] : la[comp[c]];
+      p.in[comp[c]] = static_cast<const T*>(n == 0 ? la[comp[c]] : to);
+      J.in[c] = p.in[comp[c]];
+      J.out[c] = static_cast<T*>(to);
+    }
+    // the first step's share straight into lambda, the later ones as tables
+    p.t = t;
+    if ((rc = inject_monitors<T>(p, mons, n_mon, false, g->pol, s)) != DN_OK) return rc;
+    SampleSet<T> set{};
+    unsigned char* at = ws + P.mail_bytes;
+    for (int m = 0; m < n_mon && k > 1; ++m) {
+      const BoxDev b = to_dev(mons[m].box);
+      const long long ncell = b.cells();
+      Samples<T>& q = set.s[set.n++];
+      for (int a = 0; a < 2; ++a) {
+        q.lo[a] = b.lo[1 + a];
+        q.hi[a] = b.hi[1 + a];
+      }
+      q.vec = q.lo[1] % VEC == 0 && (q.hi[1] - q.lo[1]) % VEC == 0;
+      q.buf = reinterpret_cast<T*>(at);
+      q.step_stride = (ncell * (long long)sizeof(T) + 15) / 16 * 16 / sizeof(T);
+      at += q.step_stride * sizeof(T) * k;
+      const long long blocks = (ncell * (k - 1) + 255) / 256;
+      k_add_table<T><<<(unsigned)std::min(blocks, 148LL * 16), 256, 0, s>>>(
+          q.buf, q.step_stride, k - 1, t - 1, ncell, mons[m].phase, mons[m].n_freq, mons[m].acc);
+    }
+    if (P.mail_bytes) DN_CUDA_CHECK(cudaMemsetAsync(ws, 0, P.mail_bytes, s));
+    rc = run_resident_adjoint<T>(J, set, P.S, reinterpret_cast<uint64_t*>(ws), status, s);
+    if (rc != DN_OK) return rc;
+    DN_CUDA_CHECK(cudaGetLastError());
+  }
+  *final_in_b = nsteps % 2;
+  return DN_OK;
+}
+
 }  // namespace
 }  // namespace res
 }  // namespace dn
+
+extern "C" int32_t dn_fdtd2d_adjoint_ws(const dn_grid* g, void* const la[6], void* const lb[6],
+                                        const void* ce, const dn_cpml* cpml,
+                                        const dn_curl_record* curl, double* grad_ce,
+                                        const dn_monitor* mons, int32_t n_mon, int32_t t_end,
+                                        int32_t nsteps, int32_t* status, void* stream,
+                                        int32_t* final_in_b, void* ws, int64_t ws_bytes) {
+  if (!g) return DN_EINVAL;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  unsigned char* const w = static_cast<unsigned char*>(ws);
+  if (nsteps >= dn::res::MIN_STEPS && (ws || ws_bytes == 0)) {
+    bool done = false;
+    int rc = DN_OK;
+    if (g->dtype == DN_F32)
+      rc = dn::res::adjoint_ws<float>(g, la, lb, ce, cpml, curl, grad_ce, mons, n_mon, t_end,
+                                      nsteps, status, s, final_in_b, w, ws_bytes, &done);
+    else if (g->dtype == DN_F64)
+      rc = dn::res::adjoint_ws<double>(g, la, lb, ce, cpml, curl, grad_ce, mons, n_mon, t_end,
+                                       nsteps, status, s, final_in_b, w, ws_bytes, &done);
+    if (rc != DN_OK || done) return rc;
+  }
+  return dn_fdtd2d_adjoint(g, la, lb, ce, cpml, curl, grad_ce, mons, n_mon, t_end, nsteps, status,
+                           stream, final_in_b);
+}
 
 extern "C" int64_t dn_fdtd2d_workspace_bytes(const dn_grid* g, const dn_source* src,
                                              const dn_monitor* mons, int32_t n_mon,
@@ -278,7 +408,9 @@ extern "C" int64_t dn_fdtd2d_workspace_bytes(const dn_grid* g, const dn_source* 
     return -1;
   for (int m = 0; m < n_mon; ++m)
     if (!dn::box_ok(mons[m].box, 1, g->H, g->W)) return -1;
-  return dn::res::workspace_of(dn::res::make_plan2d(g, src, mons, n_mon, nsteps));
+  return std::max(
+      dn::res::workspace_of(dn::res::make_plan2d(g, src, mons, n_mon, nsteps, false)),
+      dn::res::workspace_of(dn::res::make_plan2d(g, nullptr, mons, n_mon, nsteps, true)));
 }
 
 extern "C" int32_t dn_fdtd2d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],

@@ -67,7 +67,27 @@ struct Job {
   long long curl_stride;
 };
 
-// A box whose values of one component are stored after every step:
+// One grid's reverse sweep (TM): adjoint fields (lambda_Ez, lambda_Hx,
+// lambda_Hy); reverse step n = 0 .. nsteps-1 reads the curl record at curl - n *
+// curl_stride and adds lambda_Ez . curl to grad.
+template <typename T>
+struct AdjJob {
+  int H, W;
+  long long py;
+  const T* in[3];
+  T* out[3];
+  const T* ce;
+  const double* b[2];
+  const double* c[2];
+  double dt, dl;
+  int nsteps;
+  const T* curl;
+  long long curl_stride;
+  double* grad;
+};
+
+// A box whose values of one component are stored after every step (the reverse
+// sweep reads them instead: what is added to lambda_Ez after reverse step n):
 // buf[n * step_stride + cell], cells row-major inside the box.
 template <typename T>
 struct Samples {
@@ -92,6 +112,9 @@ struct Split {
 };
 
 // the run itself (dn_resident2d_fwd.cuh), one instantiation per source file
+template <typename T>
+int run_resident_adjoint(const AdjJob<T>& J, const SampleSet<T>& adds, const Split& S,
+                         uint64_t* mail, int* status, cudaStream_t s);
 template <typename T, int POL>
 int run_resident(const Job<T>& J, const SampleSet<T>& smps, const Split& S, uint64_t* mail,
                  int* status, cudaStream_t s);

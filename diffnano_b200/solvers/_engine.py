@@ -243,6 +243,12 @@ class Engine:
             return (_lib.DN_EX, _lib.DN_EY, _lib.DN_EZ)
         return (_lib.DN_EZ,) if self.pol == _lib.DN_TM else (_lib.DN_EX, _lib.DN_EY)
 
+    def curl_bytes(self, nslots: int) -> int:
+        """Bytes of ``curl_buffer(nslots)``."""
+        D, H, _ = self.shape3
+        ncomp = 3 if self.is3d else len(self.eps_components())
+        return ncomp * nslots * D * H * self.Wp * (4 if self.dtype == torch.float32 else 8)
+
     def curl_buffer(self, nslots: int) -> torch.Tensor:
         """``(3, nslots, D, H, Wp)`` curl storage (only the slots of the
         components that carry eps are written)."""
@@ -265,14 +271,15 @@ class Engine:
         holds the current adjoint).  Returns True when the result ends in lb."""
         L = _lib.lib()
         out = ctypes.c_int32(0)
-        fn_name = "dn_fdtd3d_adjoint" if self.is3d else "dn_fdtd2d_adjoint"
+        fn_name = "dn_fdtd3d_adjoint" if self.is3d else "dn_fdtd2d_adjoint_ws"
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device).cuda_stream
+            ws = () if self.is3d else self._workspace()
             rc = getattr(L, fn_name)(
                 ctypes.byref(self.grid), self._ptrs(la), self._ptrs(lb), self.ce.data_ptr(),
                 ctypes.byref(self.cpml), ctypes.byref(rec), grad_ce.data_ptr(), mon_arr,
                 int(n_mon), int(t_end), int(nsteps), self.status.data_ptr(),
-                ctypes.c_void_p(stream), ctypes.byref(out))
+                ctypes.c_void_p(stream), ctypes.byref(out), *ws)
         _lib.check(fn_name, rc)
         return bool(out.value)
 

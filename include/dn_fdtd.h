@@ -211,6 +211,15 @@ int32_t dn_fdtd2d_adjoint(const dn_grid* g, void* const la[6], void* const lb[6]
                           const dn_cpml* cpml, const dn_curl_record* curl, double* grad_ce,
                           const dn_monitor* mons, int32_t n_mon, int32_t t_end, int32_t nsteps,
                           int32_t* status, void* stream, int32_t* final_in_b);
+/* the 2-D sweep with a workspace (see dn_fdtd2d_run_ws; one of
+ * dn_fdtd2d_workspace_bytes serves both): TM sweeps of grids that fit on the chip
+ * run in one launch; the set that does not hold the result is left as it was,
+ * except for what the monitors add to `la` before the first step */
+int32_t dn_fdtd2d_adjoint_ws(const dn_grid* g, void* const la[6], void* const lb[6],
+                             const void* ce, const dn_cpml* cpml, const dn_curl_record* curl,
+                             double* grad_ce, const dn_monitor* mons, int32_t n_mon,
+                             int32_t t_end, int32_t nsteps, int32_t* status, void* stream,
+                             int32_t* final_in_b, void* ws, int64_t ws_bytes);
 int32_t dn_fdtd3d_adjoint(const dn_grid* g, void* const la[6], void* const lb[6], const void* ce,
                           const dn_cpml* cpml, const dn_curl_record* curl, double* grad_ce,
                           const dn_monitor* mons, int32_t n_mon, int32_t t_end, int32_t nsteps,

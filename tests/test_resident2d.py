@@ -153,3 +153,52 @@ def test_workspace_bytes_reject_invalid_input():
     assert L.dn_fdtd2d_workspace_bytes(ctypes.byref(g), None, None, 1, 10) == -1
     g.H = 0
     assert L.dn_fdtd2d_workspace_bytes(ctypes.byref(g), None, None, 0, 10) == -1
+
+
+def _sweep(eng, ws, la, lb, rec, grad, mon_arr, n_mon, t_end, T):
+    L, out = _lib.lib(), ctypes.c_int32(0)
+    args = (ctypes.byref(eng.grid), eng._ptrs(la), eng._ptrs(lb), eng.ce.data_ptr(),
+            ctypes.byref(eng.cpml), ctypes.byref(rec), grad.data_ptr(), mon_arr, n_mon, t_end, T,
+            eng.status.data_ptr(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream),
+            ctypes.byref(out))
+    if ws:
+        _lib.check("ws", L.dn_fdtd2d_adjoint_ws(*args, *eng._workspace()))
+    else:
+        _lib.check("steps", L.dn_fdtd2d_adjoint(*args))
+    eng.check_status(extra=(grad,))
+    return lb if out.value else la
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("H,W", [s for s in SHAPES if s[0] * s[1] < 500_000])
+def test_reverse_sweep(cuda, H, W, dtype):
+    """From random adjoint fields, curl terms and a running gradient, with a row
+    and a box monitor whose gradients enter before every step."""
+    f = _lib.DN_EZ
+    mons = [MonitorSpec("row", f, ((0, 1), (H // 2, H // 2 + 1), (0, W)), [1500.0, 1600.0]),
+            MonitorSpec("box", f, ((0, 1), (0, (H + 1) // 2), (W // 2, W)), [1550.0])]
+    for T in (9, 24):
+        eng = _engine(H, W, _lib.DN_TM, dtype, T + 3, mons)
+        g = torch.Generator().manual_seed(T)
+        rand = lambda *s: torch.randn(*s, dtype=torch.float64, generator=g)  # noqa: E731
+        lam, curl, grad0 = rand(6, 1, H, W), rand(T, H, W), rand(1, H, W)
+        gm = [rand(*a.shape).to(cuda) for a in eng.accs]
+        mon_arr = (_lib.DnMonitor * 2)()
+        for m in range(2):
+            ctypes.memmove(ctypes.byref(mon_arr[m]), ctypes.byref(eng.mon_arr[m]),
+                           ctypes.sizeof(_lib.DnMonitor))
+            mon_arr[m].acc = gm[m].data_ptr()
+        buf = eng.curl_buffer(T).zero_()
+        buf[0, :, 0, :, :W] = curl.to(cuda, dtype)
+        rec = eng.curl_record(buf, 2, T)
+        got = []
+        for ws in (True, False):
+            la, lb = torch.zeros_like(eng.A), torch.zeros_like(eng.A)
+            la[..., :W] = lam.to(cuda, dtype)
+            grad = torch.zeros(1, H, eng.Wp, dtype=torch.float64, device=cuda)
+            grad[..., :W] = grad0.to(cuda)
+            out = _sweep(eng, ws, la, lb, rec, grad, mon_arr, 2, T + 2, T)
+            got.append([out[c, ..., :W].clone() for c in _comps(_lib.DN_TM)] + [grad[..., :W]])
+        for a, b in zip(*got):
+            assert rel_l2(a, b) < 2 * _tol(dtype, T)
