@@ -7,16 +7,21 @@ autograd inside a custom ``autograd.Function`` (``fdtd3d.py:88-219``).  Here
 both modes are one ``torch.autograd.Function`` whose backward is the discrete
 adjoint of the kernels' own step:
 
-* forward: all T steps run in the CUDA kernels; when a gradient is needed the
-  state is copied every K steps (K = sqrt(T), or T / checkpoint_segments with
-  ``use_checkpoint``);
-* backward: for each segment, last first, the segment is replayed from its
-  checkpoint with the curl term of every step recorded, then the adjoint
-  kernel runs the segment's steps backwards, accumulating dL/d(dt/eps) in
-  FP64; dL/deps = -(dt/eps^2) dL/d(dt/eps).
+* forward: all T steps run in the CUDA kernels.  When a gradient is needed and
+  the curl terms of all T steps fit an eighth of the GPU's memory, they are
+  recorded as the steps run; else (and whenever the caller asks for
+  checkpoints) the state is copied every K steps (K = sqrt(T), or T /
+  checkpoint_segments with ``use_checkpoint``);
+* backward: with a full record, the adjoint kernel runs all steps backwards;
+  with checkpoints, each segment, last first, is replayed from its checkpoint
+  with the curl term of every step recorded and then run backwards.  Both
+  accumulate dL/d(dt/eps) in FP64; dL/deps = -(dt/eps^2) dL/d(dt/eps).
 
-Peak memory is the checkpoints (T/K states) plus one segment of curl records
-(K x 3 fields), not the T-step autograd graph.
+The full record costs one more write of the curl terms in the forward run and
+saves the replay, about a third of a gradient's time (96 x 192 x 192, 300 steps:
+142 us per step with the replay, 107 without).  Peak memory is the record, or
+the checkpoints (T/K states) plus one segment of curl records (K x 3 fields),
+not the T-step autograd graph.
 """
 
 from __future__ import annotations
@@ -27,6 +32,7 @@ from diffnano_b200 import _lib
 from diffnano_b200.solvers._common import checkpoint_interval
 
 F64 = torch.float64
+RECORD_SHARE = 1 / 8  # of the GPU's memory, for the curl terms of all steps
 
 
 def _outputs(eng, out_names):
@@ -39,18 +45,29 @@ def _outputs(eng, out_names):
 class _Runner:
     """Forward with checkpoints and the adjoint sweep for one Engine."""
 
-    def __init__(self, eng, out_names, interval: int):
+    def __init__(self, eng, out_names, interval: int, full_record: bool = False):
         self.eng = eng
         self.out_names = tuple(out_names)
         self.K = max(1, int(interval))
         self.checkpoints = {}
+        self.full_record = full_record  # try to record every step's curl terms
+        self.curl = None
 
     def forward(self, eps_dev: torch.Tensor, save: bool):
         eng = self.eng
         eng.reset()
         eng.set_eps(eps_dev)
         T, K = eng.n_steps, self.K
+        if save and self.full_record and eng.curl_bytes(T) <= RECORD_SHARE * \
+                torch.cuda.get_device_properties(eng.device).total_memory:
+            try:
+                self.curl = eng.curl_buffer(T)
+            except torch.OutOfMemoryError:
+                self.curl = None  # checkpoints need less
         t = 0
+        if self.curl is not None:
+            eng.run(0, T, record=eng.curl_record(self.curl, 0, T))
+            t = T
         while t < T:
             n = min(K, T - t)
             if save and t > 0:
@@ -96,6 +113,11 @@ class _Runner:
         n_mon = len(eng.monitors) if g_mon is not None else 0
         grad_ce = torch.zeros((D, H, eng.Wp), dtype=F64, device=eng.device)
         T, K = eng.n_steps, self.K
+        if self.curl is not None:
+            rec = eng.curl_record(self.curl, 0, T)
+            eng.adjoint(la, lb, rec, grad_ce, mon_arr, n_mon, T, T)
+            eng.check_status(extra=(grad_ce[..., :W],))
+            return grad_ce[..., :W]
         curl = eng.curl_buffer(min(K, T))
         starts = list(range(0, T, K))
         for ta in reversed(starts):
@@ -151,10 +173,10 @@ def run_forward(solver, eng, eps: torch.Tensor, out_names):
     if isinstance(out_names, str):
         out_names = (out_names,)
     needs_grad = eps.requires_grad and torch.is_grad_enabled()
-    interval = checkpoint_interval(eng.n_steps, solver.use_checkpoint or
-                                   getattr(solver, "backward", "") == "checkpoint",
-                                   solver.checkpoint_segments)
-    runner = _Runner(eng, out_names, interval if needs_grad else eng.n_steps)
+    asked = solver.use_checkpoint or getattr(solver, "backward", "") == "checkpoint"
+    interval = checkpoint_interval(eng.n_steps, asked, solver.checkpoint_segments)
+    runner = _Runner(eng, out_names, interval if needs_grad else eng.n_steps,
+                     full_record=not asked)
     if needs_grad:
         fn = _TimeReversalFDTD if getattr(solver, "backward", "auto") == "time_reversal" \
             else _FDTDAdjoint
