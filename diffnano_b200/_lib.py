@@ -160,6 +160,13 @@ SIGNATURES = {
                                   c_void_p, c_int64]),
     "dn_batch2d_forward": (c_int32, [ctypes.POINTER(DnBatch2d), c_void_p, c_void_p, c_void_p]),
     "dn_batch2d_backward": (c_int32, [ctypes.POINTER(DnBatch2d), c_void_p, c_void_p, c_void_p]),
+    "dn_batch2d_resident_bytes": (c_int64, [ctypes.POINTER(DnBatch2d),
+                                            ctypes.POINTER(DnBatch2dInst), c_int32]),
+    "dn_batch2d_resident_pack": (c_int32, [ctypes.POINTER(DnBatch2d),
+                                           ctypes.POINTER(DnBatch2dInst), c_int32, c_void_p,
+                                           c_int64, ctypes.POINTER(c_int64)]),
+    "dn_batch2d_run_resident": (c_int32, [ctypes.POINTER(DnBatch2d), c_void_p, c_void_p, c_void_p,
+                                          c_void_p, c_int64, c_int32, c_void_p, c_void_p]),
     "dn_batch2d_cluster_size": (c_int32, [ctypes.POINTER(DnBatch2d), ctypes.POINTER(DnBatch2dInst),
                                           ctypes.POINTER(c_int64)]),
     "dn_batch2d_forward_cluster": (c_int32, [ctypes.POINTER(DnBatch2d), c_void_p, c_int32,

@@ -1341,6 +1341,18 @@ int dispatch_cluster(int cl, bool db, void* table, int n_inst, long long smem, c
 }  // namespace
 }  // namespace dn
 
+namespace dn {
+// byte offset of the (sorted) instances in a packed table, -1 on invalid input
+long long batch2d_inst_offset(const dn_batch2d* cfg, const dn_batch2d_inst* insts) {
+  if (validate(cfg, insts) != DN_OK) return -1;
+  const int tt = total_tiles_of(cfg, insts);
+  if (tt < 0) return -1;
+  size_t op, os, om, oi, oe;
+  table_offsets(cfg->n_inst, tt, &op, &os, &om, &oi, &oe);
+  return (long long)oi;
+}
+}  // namespace dn
+
 extern "C" int32_t dn_batch2d_cluster_size(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                            int64_t* smem_bytes) {
   if (dn::validate(cfg, insts) != DN_OK || !smem_bytes) return -1;

@@ -1,0 +1,271 @@
+// Batched TM runs and reverse sweeps on the chip (dn_resident2d.cuh, struct
+// List): which CTA takes which bands of which grids, and the entry points.
+#include <algorithm>
+#include <cstring>
+#include <numeric>
+#include <vector>
+
+#include "dn_resident2d.cuh"
+#include "dn_sample_dft.cuh"
+
+namespace dn {
+
+long long batch2d_inst_offset(const dn_batch2d* cfg, const dn_batch2d_inst* insts);
+
+namespace res {
+namespace {
+
+// samples of one launch (more grids than fit go in further launches)
+constexpr long long GROUP_SAMPLE_BYTES = 1LL << 30;
+
+// The blob: Head | ListGrid[n_inst] | per group: start[n_cta + 1], jobs | (host
+// and device copies are the same bytes).  Grids are in the table's order.
+struct Group {
+  int first, count;           // grids
+  long long o_start, o_jobs;  // byte offsets
+  long long mail_words, sample_bytes;
+  long long max_cells;        // largest monitor
+};
+constexpr int MAX_GROUPS = 256;
+struct Head {
+  int n_inst, n_cta, R, adjoint, n_groups, pad;
+  long long inst_offset, o_grids, bytes, ws_bytes;
+  Group group[MAX_GROUPS];
+};
+
+struct Plan {
+  Head h{};
+  std::vector<ListGrid> grids;
+  std::vector<std::vector<int>> start;
+  std::vector<std::vector<ListJob>> jobs;
+};
+
+inline long long up16(long long x) { return (x + 15) / 16 * 16; }
+
+// false: some grid does not fit, or the batch is not a TM one
+bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint, Plan* P) {
+  const long long off = batch2d_inst_offset(cfg, insts);
+  if (off < 0 || cfg->pol != DN_TM) return false;
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return false;
+  const int n = cfg->n_inst, elem = cfg->dtype == DN_F32 ? 4 : 8, cols = 32 * 16 / elem;
+  std::vector<int> order(n);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(),
+                   [&](int a, int b) { return insts[a].n_steps > insts[b].n_steps; });
+  auto grid_of = [&](const dn_batch2d_inst& I, int R) {
+    ListGrid G{};
+    G.strips = (I.W + cols - 1) / cols;
+    G.groups = G.strips > MAX_WARPS
+                   ? 0 : std::min(MAX_WARPS / G.strips, std::max(1, (I.H + R - 1) / R));
+    G.bands = G.groups ? (I.H + G.groups * R - 1) / (G.groups * R) : 0;
+    return G;
+  };
+  // the fewest rows per warp for which every band has a CTA of its own, else the
+  // most that registers hold: fewer bands, less time in exchanges per cell
+  // (256^2 FP32 x 96: R = 4 20 ms, R = 2 24 ms)
+  const int r_last = adjoint ? 2 : 4;
+  int R = 1;
+  for (;; R *= 2) {
+    long long bands = 0;
+    for (int b = 0; b < n; ++b) {
+      const ListGrid G = grid_of(insts[b], R);
+      if (G.groups == 0) return false;
+      bands += G.bands;
+    }
+    if (bands <= nsm || R == r_last) break;
+  }
+  Head& h = P->h;
+  h.n_inst = n;
+  h.n_cta = nsm;
+  h.R = R;
+  h.adjoint = adjoint;
+  h.inst_offset = off;
+  long long ws = 0;
+  for (int k = 0; k < n;) {
+    if (h.n_groups == MAX_GROUPS) return false;
+    Group g{};
+    g.first = k;
+    long long mail = 0, sample = 0;
+    // each grid's bands go to the CTAs that are free first
+    std::vector<double> load(nsm, 0.0);
+    std::vector<std::vector<ListJob>> lists(nsm);
+    std::vector<int> by(nsm);
+    for (; k < n; ++k) {
+      const dn_batch2d_inst& I = insts[order[k]];
+      ListGrid G = grid_of(I, R);
+      if (G.bands > nsm) return false;
+      long long cells = 0, bytes = 0;
+      if (I.mon_comp != DN_NONE) {
+        cells = (long long)(I.mon_box.hi[1] - I.mon_box.lo[1]) *
+                (I.mon_box.hi[2] - I.mon_box.lo[2]);
+        G.stride = up16(cells * elem) / elem;
+        bytes = G.stride * elem * I.n_steps;
+      }
+      if (bytes > GROUP_SAMPLE_BYTES) return false;
+      if (k > g.first && sample + bytes > GROUP_SAMPLE_BYTES) break;
+      G.mail = mail;
+      G.sample = sample;
+      mail += (long long)G.bands * 4 * G.strips * ROW_WORDS;
+      sample += bytes;
+      g.max_cells = std::max(g.max_cells, cells);
+      P->grids.push_back(G);
+      std::iota(by.begin(), by.end(), 0);
+      std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return load[a] < load[b]; });
+      const double end = load[by[G.bands - 1]] + I.n_steps;
+      for (int b = 0; b < G.bands; ++b) {
+        lists[by[b]].push_back({k, b});
+        load[by[b]] = end;
+      }
+    }
+    g.count = k - g.first;
+    g.mail_words = mail;
+    g.sample_bytes = sample;
+    ws = std::max(ws, mail * 8 + sample);
+    std::vector<int> start(nsm + 1, 0);
+    std::vector<ListJob> jobs;
+    for (int c = 0; c < nsm; ++c) {
+      jobs.insert(jobs.end(), lists[c].begin(), lists[c].end());
+      start[c + 1] = (int)jobs.size();
+    }
+    P->start.push_back(start);
+    P->jobs.push_back(jobs);
+    h.group[h.n_groups++] = g;
+  }
+  long long at = up16(sizeof(Head));
+  h.o_grids = at;
+  at += up16((long long)n * sizeof(ListGrid));
+  for (int g = 0; g < h.n_groups; ++g) {
+    h.group[g].o_start = at;
+    at += up16((nsm + 1) * sizeof(int));
+    h.group[g].o_jobs = at;
+    at += up16((long long)P->jobs[g].size() * sizeof(ListJob));
+  }
+  h.bytes = at;
+  h.ws_bytes = ws;
+  return true;
+}
+
+// running DFTs of a group's monitors, one grid per blockIdx.y
+template <typename T>
+__global__ void __launch_bounds__(DFT_WARPS * 32)
+    k_list_dft(const dn_batch2d_inst* insts, const ListGrid* grids, unsigned char* samples,
+               int first, const int* status) {
+  if (status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;
+  const dn_batch2d_inst& I = insts[first + blockIdx.y];
+  const ListGrid& G = grids[first + blockIdx.y];
+  if (I.mon_comp == DN_NONE) return;
+  const long long ncell = (long long)(I.mon_box.hi[1] - I.mon_box.lo[1]) *
+                          (I.mon_box.hi[2] - I.mon_box.lo[2]);
+  if (blockIdx.x * 32LL >= ncell) return;
+  sample_dft<T>(reinterpret_cast<const T*>(samples + G.sample), G.stride, I.n_steps, ncell, I.phase,
+                I.n_freq, I.acc);
+}
+
+// what a group's monitors add in the reverse sweep: before the first step straight
+// into lambda, for the later ones a table; one grid per blockIdx.y
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_list_adds(const dn_batch2d_inst* insts, const ListGrid* grids, unsigned char* samples,
+                int first) {
+  const dn_batch2d_inst& I = insts[first + blockIdx.y];
+  const ListGrid& G = grids[first + blockIdx.y];
+  if (I.mon_comp == DN_NONE || I.gmon == nullptr) return;
+  const int bw = I.mon_box.hi[2] - I.mon_box.lo[2];
+  const long long ncell = (long long)(I.mon_box.hi[1] - I.mon_box.lo[1]) * bw;
+  T* table = reinterpret_cast<T*>(samples + G.sample);
+  T* lam = static_cast<T*>(I.lam[I.n_steps & 1][0]);
+  for (long long e = blockIdx.x * 256LL + threadIdx.x; e < ncell * I.n_steps;
+       e += gridDim.x * 256LL) {
+    const long long n = e / ncell, cell = e - n * ncell;
+    const T v = add_of<T>(cell, ncell, I.n_steps - 1 - n, I.phase, I.n_freq, I.gmon);
+    if (n == 0)
+      lam[(I.mon_box.lo[1] + cell / bw) * I.pitch + I.mon_box.lo[2] + cell % bw] += v;
+    else
+      table[(n - 1) * G.stride + cell] = v;
+  }
+}
+
+template <typename T>
+int run_groups(const Head& h, bool record, unsigned char* table, unsigned char* blob,
+               unsigned char* ws, int* status, cudaStream_t s) {
+  const dn_batch2d_inst* insts = reinterpret_cast<const dn_batch2d_inst*>(table + h.inst_offset);
+  const ListGrid* grids = reinterpret_cast<const ListGrid*>(blob + h.o_grids);
+  for (int q = 0; q < h.n_groups; ++q) {
+    const Group& g = h.group[q];
+    List L{insts,
+           grids,
+           reinterpret_cast<const ListJob*>(blob + g.o_jobs),
+           reinterpret_cast<const int*>(blob + g.o_start),
+           reinterpret_cast<uint64_t*>(ws),
+           ws + g.mail_words * 8};
+    DN_CUDA_CHECK(cudaMemsetAsync(ws, 0, (size_t)g.mail_words * 8, s));
+    const unsigned cells = (unsigned)((g.max_cells + 31) / 32);
+    if (h.adjoint && cells) {
+      k_list_adds<T><<<dim3(64, g.count), 256, 0, s>>>(insts, grids, L.samples, g.first);
+      DN_CUDA_CHECK(cudaGetLastError());
+    }
+    const int rc = run_resident_list<T>(L, h.adjoint, record, h.R, h.n_cta, status, s);
+    if (rc != DN_OK) return rc;
+    if (!h.adjoint && cells) {
+      k_list_dft<T><<<dim3(cells, g.count), DFT_WARPS * 32, 0, s>>>(insts, grids, L.samples,
+                                                                    g.first, status);
+      DN_CUDA_CHECK(cudaGetLastError());
+    }
+  }
+  return DN_OK;
+}
+
+}  // namespace
+}  // namespace res
+}  // namespace dn
+
+extern "C" int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                             int32_t adjoint) {
+  if (!cfg || !insts) return -1;
+  dn::res::Plan P;
+  return dn::res::make_plan(cfg, insts, adjoint != 0, &P) ? P.h.bytes : 0;
+}
+
+extern "C" int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                            int32_t adjoint, void* host_plan, int64_t bytes,
+                                            int64_t* ws_bytes) {
+  if (!cfg || !insts || !host_plan || !ws_bytes) return DN_EINVAL;
+  dn::res::Plan P;
+  if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P)) return DN_EUNSUPPORTED;
+  if (bytes < P.h.bytes) return DN_EINVAL;
+  unsigned char* b = static_cast<unsigned char*>(host_plan);
+  std::memset(b, 0, (size_t)P.h.bytes);
+  std::memcpy(b, &P.h, sizeof(P.h));
+  std::memcpy(b + P.h.o_grids, P.grids.data(), P.grids.size() * sizeof(dn::res::ListGrid));
+  for (int g = 0; g < P.h.n_groups; ++g) {
+    std::memcpy(b + P.h.group[g].o_start, P.start[g].data(), P.start[g].size() * sizeof(int));
+    std::memcpy(b + P.h.group[g].o_jobs, P.jobs[g].data(),
+                P.jobs[g].size() * sizeof(dn::res::ListJob));
+  }
+  *ws_bytes = P.h.ws_bytes;
+  return DN_OK;
+}
+
+extern "C" int32_t dn_batch2d_run_resident(const dn_batch2d* cfg, void* dev_table,
+                                           const void* host_plan, void* dev_plan, void* ws,
+                                           int64_t ws_bytes, int32_t record, int32_t* status,
+                                           void* stream) {
+  if (!cfg || !dev_table || !host_plan || !dev_plan ||
+      ((reinterpret_cast<uintptr_t>(dev_table) | reinterpret_cast<uintptr_t>(dev_plan) |
+        reinterpret_cast<uintptr_t>(ws)) & 15))
+    return DN_EINVAL;
+  const dn::res::Head& h = *static_cast<const dn::res::Head*>(host_plan);
+  if (cfg->n_inst != h.n_inst || cfg->pol != DN_TM || ws_bytes < h.ws_bytes || (h.ws_bytes && !ws))
+    return DN_EINVAL;
+  unsigned char *t = static_cast<unsigned char*>(dev_table),
+                *b = static_cast<unsigned char*>(dev_plan), *w = static_cast<unsigned char*>(ws);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (cfg->dtype == DN_F32)
+    return dn::res::run_groups<float>(h, record != 0, t, b, w, status, s);
+  if (cfg->dtype == DN_F64)
+    return dn::res::run_groups<double>(h, record != 0, t, b, w, status, s);
+  return DN_EINVAL;
+}

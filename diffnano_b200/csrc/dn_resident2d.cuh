@@ -111,6 +111,33 @@ struct Split {
   int cluster;  // bands exchange rows through shared memory (else through global memory)
 };
 
+// Many grids in one cooperative launch: every CTA takes the (grid, band) pairs of
+// its list in order.  Bands of a grid wait for one another, so all lists keep one
+// order of the grids: the bands of the first unfinished grid are always next on
+// their CTAs.
+struct ListGrid {
+  int strips, groups, bands;
+  long long mail;    // 64-bit words from the start of the mailboxes
+  long long sample;  // bytes from the start of the samples
+  long long stride;  // elements between two steps' samples
+};
+struct ListJob {
+  int grid, band;
+};
+struct List {
+  const dn_batch2d_inst* inst;
+  const ListGrid* grids;
+  const ListJob* jobs;
+  const int* start;  // per CTA, its first job (and one past the last CTA's last)
+  uint64_t* mail;
+  unsigned char* samples;
+};
+
+// forward (adjoint = false) or reverse sweep of TM grids, R rows per warp
+template <typename T>
+int run_resident_list(const List& L, bool adjoint, bool record, int R, int n_cta, int* status,
+                      cudaStream_t s);
+
 // the run itself (dn_resident2d_fwd.cuh), one instantiation per source file
 template <typename T>
 int run_resident_adjoint(const AdjJob<T>& J, const SampleSet<T>& adds, const Split& S,

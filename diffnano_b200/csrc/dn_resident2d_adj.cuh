@@ -145,7 +145,7 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
   auto advance = [&](auto par_c, int n) -> bool {
     constexpr int PAR = decltype(par_c)::value;
     constexpr int NXT = PAR ^ 1;
-    step(PAR, n);
+    if (K.active) step(PAR, n);
     if (n + 1 == J.nsteps) return false;
     if (add_mask) {
 #pragma unroll 1
@@ -169,10 +169,12 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
         }
       }
     }
+    if (K.active) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) u[r] = mulv<T>(coef_e(r), e[r]);
-    K.post(NXT, n, u);
-    K.publish(NXT, u);
+      for (int r = 0; r < R; ++r) u[r] = mulv<T>(coef_e(r), e[r]);
+      K.post(NXT, n, u);
+      K.publish(NXT, u);
+    }
     __syncthreads();
     const bool go = K.gather(NXT, n, u_up, u_dn);
     if (ia <= 1) {  // row ia-1 = 0 has no weight on its own u; row -1 does not exist

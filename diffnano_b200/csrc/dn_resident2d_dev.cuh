@@ -312,6 +312,7 @@ struct Block {
   unsigned char* smem;
   int* status;
   int lane, w, strip, group, ia0, ia, j0, jv;
+  bool active;  // has a block (a CTA may have more warps than a grid's bands use)
   bool live, any, full;
   bool first_row, last_row, first_col, last_col;
   bool band_up, band_dn;  // rows from and to another CTA
@@ -345,7 +346,8 @@ struct Block {
     ia = ia0 + group * R;
     j0 = strip * COLS;
     jv = j0 + lane * VEC;
-    live = ia < H;
+    active = group < S.groups;
+    live = active && ia < H;
     any = jv < W;
     full = jv + VEC <= W;
     first_row = ia == 0;

@@ -192,7 +192,7 @@ __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int ba
     constexpr int PAR = decltype(par_c)::value;
     constexpr int NXT = PAR ^ 1;
     const int t = J.t0 + n;
-    step(PAR, n);
+    if (K.active) step(PAR, n);
     if (src_rows) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -203,7 +203,7 @@ __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int ba
     if (more) {
       if (has_ghosts) ghosts();
       K.post(NXT, n, f);
-      K.publish(NXT, f);
+      if (K.active) K.publish(NXT, f);
     }
     if (SMP && smp_mask) {
 #pragma unroll 1

@@ -7,7 +7,11 @@ wavelength sweeps -- of different sizes and step counts.  ``FDTDBatch2D``
 advances all of them in one persistent cooperative kernel
 (``dn_batch2d_forward``) and differentiates all of them in a second one
 (``dn_batch2d_backward``: checkpoint-segment replay + reverse steps), with the
-same step arithmetic as the single-grid kernels.  Each instance is described
+same step arithmetic as the single-grid kernels.  TM batches whose grids fit on
+the chip run grid by grid with the fields in registers instead
+(``dn_batch2d_run_resident``): always without a gradient, and with one where the
+curl terms of all steps fit an eighth of the GPU's memory (and no
+``checkpoint_interval`` was asked for).  Each instance is described
 by the reference's own constructor arguments and source dict, plus one DFT
 line/point/box monitor on its injected field.
 
@@ -16,9 +20,9 @@ line/point/box monitor on its injected field.
 CUDA graph and replays it when the same batch is solved repeatedly (design
 iterations).  The tile height is
 chosen by ``autotune_tile_rows`` (measured, cached per device and batch
-signature).  Gradient-free solves of grids that fit a thread-block cluster's
-shared memory run one cluster per grid (``dn_batch2d_forward_cluster``) unless
-``cluster=False``; large batches stream faster through the persistent kernel.
+signature).  Other gradient-free solves of grids that fit a thread-block
+cluster's shared memory run one cluster per grid (``dn_batch2d_forward_cluster``)
+unless ``cluster=False``.
 Batches of identical grids (same shape, steps, time step, wavelength and
 monitor) keep their fields, coefficients and monitor sums in batch-wide
 tensors, so eps upload, reset and outputs are one tensor operation each.
@@ -40,6 +44,7 @@ from diffnano_b200.solvers import _setup
 from diffnano_b200.solvers._engine import compute_device, padded_width
 
 F64 = torch.float64
+RECORD_SHARE = 1 / 8  # of the GPU's memory, for the curl terms of all steps
 
 
 @dataclass
@@ -68,7 +73,7 @@ class _Inst:
     """Device buffers of one instance."""
 
     def __init__(self, spec: BatchInstance, pol: int, dtype, dev, K: int, grad: bool,
-                 shared: dict | None = None, views: tuple | None = None):
+                 shared: dict | None = None, views: tuple | None = None, record: bool = False):
         H, W = spec.grid_shape
         self.spec, self.H, self.W = spec, H, W
         self.Wp = padded_width(W)
@@ -106,10 +111,14 @@ class _Inst:
             self.acc = views[2] if views is not None else \
                 torch.zeros((self.nf, cells, 2), dtype=F64, device=dev)
         self.grad_enabled = grad
-        nck = max(0, math.ceil(T / K) - 1)
-        self.ckpt = torch.zeros((max(1, nck), 3, H, self.Wp), **kw) if grad else None
+        # record: the curl terms of all steps, no checkpoints
+        nck = 0 if record else max(0, math.ceil(T / K) - 1)
+        self.ckpt = torch.zeros((max(1, nck), 3, H, self.Wp), **kw) if grad and not record else None
         ncurl = 1 if pol == _lib.DN_TM else 2
-        self.curl = torch.zeros((min(K, T), ncurl, H, self.Wp), **kw) if grad else None
+        self.curl = None
+        if grad:
+            make = torch.empty if record else torch.zeros
+            self.curl = make((T if record else min(K, T), ncurl, H, self.Wp), **kw)
         self.lam = torch.zeros((2, 3, H, self.Wp), **kw) if grad else None
         self.grad = torch.zeros((H, self.Wp), dtype=F64, device=dev) if grad else None
         self.gmon = None
@@ -138,7 +147,8 @@ class _Inst:
             s.mon_box = _lib.box([a for a, _ in self.mon_box], [b for _, b in self.mon_box])
             s.n_freq, s.phase, s.acc = self.nf, self.phase.data_ptr(), self.acc.data_ptr()
         if self.grad_enabled:
-            s.ckpt, s.curl, s.grad = self.ckpt.data_ptr(), self.curl.data_ptr(), self.grad.data_ptr()
+            s.ckpt = self.ckpt.data_ptr() if self.ckpt is not None else None
+            s.curl, s.grad = self.curl.data_ptr(), self.grad.data_ptr()
         s.gmon = self.gmon.data_ptr() if self.gmon is not None else None
         return s
 
@@ -162,12 +172,13 @@ class FDTDBatch2D:
     polarization : "TM" or "TE"
     dtype : torch.float32 (default) or torch.float64
     device : CUDA device to run on
-    checkpoint_interval : steps between stored states for the adjoint
-        (default sqrt of the longest step count)
+    checkpoint_interval : steps between stored states for the adjoint (default:
+        sqrt of the longest step count, or no stored states at all where the
+        curl terms of all steps can be recorded)
     tile_rows : 8, 16 or 32; None lets ``autotune_tile_rows`` choose
-    cluster : gradient-free solves with each grid in one 16-CTA thread-block
-        cluster: None = when every grid fits, False = never, True = always
-        (error if a grid does not fit)
+    cluster : gradient-free solves that do not run resident, with each grid in
+        one 16-CTA thread-block cluster: None = when every grid fits, False =
+        never, True = always (error if a grid does not fit)
     """
 
     def __init__(self, instances, polarization: str = "TM", dtype=torch.float32,
@@ -186,6 +197,11 @@ class FDTDBatch2D:
         T = max(s.n_steps for s in self.specs)
         self.K = int(checkpoint_interval or max(1, math.ceil(math.sqrt(T))))
         self.tile_rows = tile_rows
+        self._auto_rows = tile_rows is None
+        self._asked_checkpoints = checkpoint_interval is not None
+        self._record = False
+        self._plans: dict = {}  # adjoint? -> (host plan, device plan, workspace bytes)
+        self._ws = None
         self._insts = None
         self._stack = None
         self._grad_alloc = None
@@ -206,16 +222,68 @@ class FDTDBatch2D:
     def _build(self, grad: bool):
         if self._insts is not None and self._grad_alloc == grad:
             return
-        shared: dict = {}
+        self._insts, self._record, self._plans = None, False, {}
         views = self._stacked_views()
-        self._insts = [_Inst(s, self.pol, self.dtype, self.device, self.K, grad, shared,
-                             None if views is None else views[n])
-                       for n, s in enumerate(self.specs)]
+        if grad and self._can_record():
+            try:
+                self._make_insts(grad, views, record=True)
+                self._record = True
+            except torch.OutOfMemoryError:
+                self._insts = None  # checkpoints need less
+        if self._insts is None:
+            self._make_insts(grad, views, record=False)
         self._grad_alloc = grad
         self._graph = None
-        if self.tile_rows is None:
+        if self._auto_rows:
+            self.tile_rows = 16
+        self._plan_resident()
+        if self._record and (False not in self._plans or True not in self._plans):
+            self._record = False  # some grid does not fit on the chip
+            self._make_insts(grad, views, record=False)
+        if self._auto_rows and not self.uses_resident(True, grad):
             self.tile_rows = autotune_tile_rows(self)
         self._pack()
+
+    def _make_insts(self, grad: bool, views, record: bool) -> None:
+        shared: dict = {}
+        self._insts = [_Inst(s, self.pol, self.dtype, self.device, self.K, grad, shared,
+                             None if views is None else views[n], record)
+                       for n, s in enumerate(self.specs)]
+
+    def _can_record(self) -> bool:
+        """Whether the curl terms of all steps may be recorded: a TM batch, no
+        checkpoints asked for, within their share of the memory."""
+        if self.pol != _lib.DN_TM or self._asked_checkpoints:
+            return False
+        size = 4 if self.dtype == torch.float32 else 8
+        need = sum(s.n_steps * s.grid_shape[0] * padded_width(s.grid_shape[1]) for s in self.specs)
+        total = torch.cuda.get_device_properties(self.device).total_memory
+        return need * size <= RECORD_SHARE * total
+
+    def _plan_resident(self) -> None:
+        """Plans of the resident forward run and (recorded) reverse sweep, where
+        the batch can run that way."""
+        L = _lib.lib()
+        arr = (_lib.DnBatch2dInst * len(self._insts))(*[i.struct(self.pol) for i in self._insts])
+        cfg = self._cfg(self.tile_rows, len(self._insts), 0)
+        with torch.cuda.device(self.device):
+            for adjoint in ((False, True) if self._record else (False,)):
+                n = int(L.dn_batch2d_resident_bytes(ctypes.byref(cfg), arr, int(adjoint)))
+                if n <= 0:
+                    continue
+                host, ws = (ctypes.c_ubyte * n)(), ctypes.c_int64(0)
+                _lib.check("dn_batch2d_resident_pack", L.dn_batch2d_resident_pack(
+                    ctypes.byref(cfg), arr, int(adjoint), host, n, ctypes.byref(ws)))
+                dev = torch.frombuffer(bytearray(host), dtype=torch.uint8).to(self.device)
+                self._plans[adjoint] = (host, dev, int(ws.value))
+        need = max((p[2] for p in self._plans.values()), default=0)
+        if self._ws is None or self._ws.numel() < need:
+            self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+
+    def uses_resident(self, fwd: bool, grad: bool) -> bool:
+        """Whether a forward (with or without gradient) or backward run keeps the
+        grids on the chip."""
+        return (not fwd) in self._plans and (self._record or not grad)
 
     def _stacked_views(self):
         """Uniform batches (every instance with the same grid, step count, time
@@ -272,14 +340,22 @@ class FDTDBatch2D:
         self.table = torch.frombuffer(bytearray(host), dtype=torch.uint8).to(self.device)
 
     def uses_cluster(self, grad: bool) -> bool:
-        """Whether a forward with / without gradient runs the cluster kernel."""
+        """Whether the batch fits the cluster kernel and may use it for a forward with /
+        without gradient (a resident plan comes first)."""
         return (not grad) and self.cluster is not False and self._cluster[0] > 0
 
     def _launch(self, fwd: bool, grad: bool = True):
         L = _lib.lib()
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device).cuda_stream
-            if fwd and self.uses_cluster(grad):
+            if self.uses_resident(fwd, grad):
+                fn = "dn_batch2d_run_resident"
+                host, plan, _ = self._plans[not fwd]
+                rc = L.dn_batch2d_run_resident(
+                    ctypes.byref(self.cfg), self.table.data_ptr(), host, plan.data_ptr(),
+                    self._ws.data_ptr() if self._ws.numel() else None, self._ws.numel(), int(grad),
+                    self.status.data_ptr(), ctypes.c_void_p(stream))
+            elif fwd and self.uses_cluster(grad):
                 fn = "dn_batch2d_forward_cluster"
                 rc = L.dn_batch2d_forward_cluster(ctypes.byref(self.cfg), self.table.data_ptr(),
                                                   self._cluster[0], self._cluster[1],
@@ -535,7 +611,8 @@ def autotune_tile_rows(batch: FDTDBatch2D, candidates=(8, 16, 32), probe_steps: 
         b = FDTDBatch2D(probe, "TM" if batch.pol == _lib.DN_TM else "TE", batch.dtype,
                         batch.device, tile_rows=rows)
         eps = [torch.full(s.grid_shape, 2.0, dtype=F64) for s in probe]
-        b.run_forward(eps)  # warm-up
+        b.run_forward(eps)  # warm-up (and the device table)
+        b._launch(True)
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record()
         b._launch(True)

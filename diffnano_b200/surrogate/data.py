@@ -103,9 +103,6 @@ class FDTDLabeler:
 
     def _solver(self, n: int) -> FDTDBatch2D:
         if self._batch is None or self._n != n:
-            # a chunk of 2048 256^2 grids streams ~3.7 GB per step: the persistent
-            # strip-march kernel (32-row tiles) labels it faster than one
-            # thread-block cluster per grid (129 vs 118 Gcell/s, identical DFTs)
             self._batch = FDTDBatch2D([self.setup.instance() for _ in range(n)], "TM",
                                       torch.float32, self.device, tile_rows=32, cluster=False)
             self._n = n

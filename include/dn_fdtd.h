@@ -313,6 +313,28 @@ int32_t dn_batch2d_cluster_size(const dn_batch2d* cfg, const dn_batch2d_inst* in
 int32_t dn_batch2d_forward_cluster(const dn_batch2d* cfg, void* dev_table, int32_t cluster,
                                    int64_t smem_bytes, void* stream);
 
+/* TM batches with every grid held on the chip while its steps run: the grids'
+ * bands of rows are dealt to the SMs by a plan, all steps of a grid run without
+ * leaving registers (as dn_fdtd2d_run_ws), in a few launches for the whole batch.
+ * Same table and results as dn_batch2d_forward / dn_batch2d_backward, with these
+ * differences: the fields start from f[0], no checkpoints are written; with
+ * `record` the forward run stores the curl terms of all steps (curl is
+ * [n_steps][H*pitch]), and the reverse sweep (a plan made with adjoint = 1) reads
+ * them, so it needs no replay.
+ * dn_batch2d_resident_bytes: size of a plan, 0 when the batch has to go the other
+ * way (TE, a grid that does not fit), -1 on invalid input.
+ * dn_batch2d_resident_pack writes the plan into host memory; the caller copies it
+ * to the device and passes both copies.  `ws`: device workspace of *ws_bytes
+ * (contents irrelevant), 16-byte aligned; runs that share one must not overlap. */
+int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                  int32_t adjoint);
+int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                 int32_t adjoint, void* host_plan, int64_t bytes,
+                                 int64_t* ws_bytes);
+int32_t dn_batch2d_run_resident(const dn_batch2d* cfg, void* dev_table, const void* host_plan,
+                                void* dev_plan, void* ws, int64_t ws_bytes, int32_t record,
+                                int32_t* status, void* stream);
+
 /* Diagnostic, no reference counterpart: runs the persistent kernels' grid
  * barrier alone, `rounds` times, on `n_ctas` one-warp CTAs (at most one per
  * SM), waiting for n_ctas + `missing` arrivals with at most `spin_limit`
