@@ -45,7 +45,7 @@ typedef struct dn_density {
 
 /* filtered = filter(rho); eps = lo + (hi - lo) * project(filtered).  work,
  * filtered and eps each hold n_layers*H*W floats; keep `filtered` for the
- * backward pass. */
+ * backward pass.  An output may be the input's buffer (work then holds a copy). */
 int32_t dn_density_forward(const dn_density* d, const float* rho, float* work, float* filtered,
                            float* eps, void* stream);
 /* drho = filter(d eps * (hi - lo) * project'(filtered)); work as above. */
