@@ -284,11 +284,7 @@ __global__ void k_monitor_adjoint(AdjParams<T> p, MonDev m) {
   const double* ph = m.phase + (long long)p.t * m.nf * 2;
   for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < n;
        cell += (long long)gridDim.x * blockDim.x) {
-    double g = 0.0;
-    for (int f = 0; f < m.nf; ++f) {
-      const double* a = m.acc + ((long long)f * n + cell) * 2;
-      g = fma(a[0], ph[2 * f], fma(a[1], ph[2 * f + 1], g));
-    }
+    const double g = monitor_grad(m, ph, cell);
     const long long nx = m.box.nx(), ny = m.box.ny();
     const int k = m.box.lo[2] + (int)(cell % nx);
     const int j = m.box.lo[1] + (int)((cell / nx) % ny);
@@ -355,24 +351,33 @@ template int build_adj_params<double>(bool, const dn_grid*, void* const*, void* 
                                       const void*, const dn_cpml*, const dn_curl_record*, double*,
                                       int, int, int*, AdjParams<double>*);
 
+template <typename T>
+int monitor_dev(const AdjParams<T>& p, const dn_monitor& M, bool is3d, int pol, MonDev* out) {
+  if (M.component < 0 || M.component > 5 || !((used_mask(is3d, pol) >> M.component) & 1u))
+    return DN_EINVAL;
+  if (!box_ok(M.box, p.D, p.H, p.W) || M.n_freq < 1 || M.n_freq > DN_MAX_FREQS || !M.phase ||
+      !M.acc)
+    return DN_EINVAL;
+  out->comp = M.component;
+  out->nf = M.n_freq;
+  out->box = to_dev(M.box);
+  out->ncell = out->box.cells();
+  out->phase = M.phase;
+  out->acc = M.acc;
+  return DN_OK;
+}
+
+template int monitor_dev<float>(const AdjParams<float>&, const dn_monitor&, bool, int, MonDev*);
+template int monitor_dev<double>(const AdjParams<double>&, const dn_monitor&, bool, int, MonDev*);
+
 // monitor-gradient injection for one adjoint step (shared with 3-D)
 template <typename T>
 int inject_monitors(const AdjParams<T>& p, const dn_monitor* mons, int n_mon, bool is3d,
                     int pol, cudaStream_t s) {
-  const unsigned used = used_mask(is3d, pol);
   for (int m = 0; m < n_mon; ++m) {
-    const dn_monitor& M = mons[m];
-    if (M.component < 0 || M.component > 5 || !((used >> M.component) & 1u)) return DN_EINVAL;
-    if (!box_ok(M.box, p.D, p.H, p.W) || M.n_freq < 1 || M.n_freq > DN_MAX_FREQS || !M.phase ||
-        !M.acc)
-      return DN_EINVAL;
     MonDev md;
-    md.comp = M.component;
-    md.nf = M.n_freq;
-    md.box = to_dev(M.box);
-    md.ncell = md.box.cells();
-    md.phase = M.phase;
-    md.acc = M.acc;
+    const int rc = monitor_dev(p, mons[m], is3d, pol, &md);
+    if (rc != DN_OK) return rc;
     const int threads = 256;
     const long long blocks = (md.ncell + threads - 1) / threads;
     k_monitor_adjoint<T><<<(unsigned)(blocks < 1024 ? blocks : 1024), threads, 0, s>>>(p, md);

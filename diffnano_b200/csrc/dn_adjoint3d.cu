@@ -41,6 +41,39 @@ struct AdjCfg {
   using L = Layout<T, NRING_A, NTILE_A, S>;
 };
 
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+
+template <typename T>
+__device__ __forceinline__ bool any_monitor(const AdjParams<T>& p, int i) {
+  bool any = false;
+#pragma unroll
+  for (int m = 0; m < DN_MAX_MONITORS; ++m) any |= m < p.n_mon && p.mon[m].box.has_plane(i);
+  return any;
+}
+
+// The monitors' gradients of step t - 1 on one cell's stored fields, in monitor
+// order (a launch of its own per monitor and step took 3.3 us and a launch gap).
+template <typename T>
+__device__ __forceinline__ void inject_cell(const AdjParams<T>& p, int i, int j, int k, T& ex, T& ey,
+                                            T& ez, T& hx, T& hy, T& hz) {
+#pragma unroll
+  for (int m = 0; m < DN_MAX_MONITORS; ++m) {
+    if (m >= p.n_mon) break;
+    const MonDev& M = p.mon[m];
+    if (!M.box.contains(i, j, k)) continue;
+    const T g = static_cast<T>(
+        monitor_grad(M, M.phase + (long long)(p.t - 1) * M.nf * 2, M.box.offset(i, j, k)));
+    const int c = M.comp;
+    ex = c == DN_EX ? add_rn(ex, g) : ex;
+    ey = c == DN_EY ? add_rn(ey, g) : ey;
+    ez = c == DN_EZ ? add_rn(ez, g) : ez;
+    hx = c == DN_HX ? add_rn(hx, g) : hx;
+    hy = c == DN_HY ? add_rn(hy, g) : hy;
+    hz = c == DN_HZ ? add_rn(hz, g) : hz;
+  }
+}
+
 template <typename T, int AXES>
 __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     k_adj3d(const AdjParams<T> p, const __grid_constant__ TmapSet tm, const Plan plan) {
@@ -187,6 +220,7 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
   // ---- march -----------------------------------------------------------------
   for (int i = z0; i < z1; ++i) {
     const bool has_next = (i + 1 < D);
+    if (i == max(z0, z1 - 2)) pdl_release();
     if ((i == 0 && !wait_full(q)) || (has_next && !wait_full(q + 1))) {
       fail();
       return;
@@ -243,6 +277,7 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     const T hvyk0 = __shfl_sync(FULL_MASK, hvyk, 0), hvyk1 = __shfl_sync(FULL_MASK, hvyk, 1);
     const T hvzk0 = __shfl_sync(FULL_MASK, hvzk, 0), hvzk1 = __shfl_sync(FULL_MASK, hvzk, 1);
 
+    const bool special = any_monitor(p, i);
     // ---- previous adjoint fields of rows ja, ja+1 ---------------------------
     const T* ct = sm.tile_arr(q, NRING_A, 0) + (2 * w) * TX + lane;
     constexpr int TE = L::TILE_ARR / (int)sizeof(T);
@@ -269,21 +304,23 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
         const T ex_b = AXES == DN_AXES_REFERENCE ? bJ[r] * bK : bJ[r] * bI;
         const T ey_b = AXES == DN_AXES_REFERENCE ? bK * bJ[r] : bI * bK;
         const T ez_b = bK * bJ[r];
-        const T nlex = ex_b * lex + (vyi - pvyi[r - 1]) - (vzj - vzj_m);
-        const T nley = ey_b * ley - (vxi - pvxi[r - 1]) + (vzk - vzk_m);
-        const T nlez = ez_b * lez + (vxj - vxj_m) - (vyk - vyk_m);
+        T nlex = ex_b * lex + (vyi - pvyi[r - 1]) - (vzj - vzj_m);
+        T nley = ey_b * ley - (vxi - pvxi[r - 1]) + (vzk - vzk_m);
+        T nlez = ez_b * lez + (vxj - vxj_m) - (vyk - vyk_m);
         const long long o = o_plane + (r - 1) * py;
         const int et = (r - 1) * TX;
         const double gsum = static_cast<double>(lex) * static_cast<double>(ct[et]) +
                             static_cast<double>(ley) * static_cast<double>(ct[TE + et]) +
                             static_cast<double>(lez) * static_cast<double>(ct[2 * TE + et]);
         p.grad[o] = gpre[r - 1] + gsum;
+        T nlhx = bJ[r] * LHx[r], nlhy = hy_b * LHy[r], nlhz = bK * LHz[r];
+        if (special) inject_cell(p, i, j, k, nlex, nley, nlez, nlhx, nlhy, nlhz);
         p.out[DN_EX][o] = nlex;
         p.out[DN_EY][o] = nley;
         p.out[DN_EZ][o] = nlez;
-        p.out[DN_HX][o] = bJ[r] * LHx[r];
-        p.out[DN_HY][o] = hy_b * LHy[r];
-        p.out[DN_HZ][o] = bK * LHz[r];
+        p.out[DN_HX][o] = nlhx;
+        p.out[DN_HY][o] = nlhy;
+        p.out[DN_HZ][o] = nlhz;
       }
       pvxi[r - 1] = vxi;
       pvyi[r - 1] = vyi;
@@ -324,15 +361,23 @@ int launch_adj(AdjParams<T> p, void* const la[6], void* const lb[6], const dn_gr
   auto kern = k_adj3d<T, AXES>;
   DN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
+  for (int m = 0; m < n_mon && nsteps > 0; ++m)
+    if ((rc = monitor_dev(p, mons[m], true, 0, &p.mon[m])) != DN_OK) return rc;
   for (int n = 0; n < nsteps; ++n) {
     const bool even = (n % 2) == 0;
     for (int c = 0; c < 6; ++c) {
       p.in[c] = static_cast<const T*>(even ? la[c] : lb[c]);
       p.out[c] = static_cast<T*>(even ? lb[c] : la[c]);
     }
+    // the first step's monitor gradients go in ahead of it, those of each further
+    // one with the stores of the step before
     p.t = t_end - 1 - n;
-    if (n_mon > 0 && (rc = inject_monitors<T>(p, mons, n_mon, true, 0, s)) != DN_OK) return rc;
-    kern<<<(unsigned)nctas, NT, smem, s>>>(p, even ? ta : tb, plan);
+    if (n == 0 && n_mon > 0 && (rc = inject_monitors<T>(p, mons, n_mon, true, 0, s)) != DN_OK)
+      return rc;
+    p.n_mon = n + 1 < nsteps ? n_mon : 0;
+    if ((rc = launch_chained(kern, (unsigned)nctas, NT, smem, s, n > 0, p, even ? ta : tb,
+                             plan)) != DN_OK)
+      return rc;
   }
   DN_CUDA_CHECK(cudaGetLastError());
   return DN_OK;

@@ -99,6 +99,14 @@ __device__ __forceinline__ bool any_special(const StepParams<T>& p, int i) {
   return any;
 }
 
+// Dependent launches: let the stream's next kernel come up and prepare while this one
+// ends; wait until everything the stream's earlier kernels wrote is there.  A
+// kernel launched without the attribute passes both at once.
+__device__ __forceinline__ void pdl_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------
 // mbarrier / TMA PTX wrappers (sm_90+; used here on sm_100a)
 // ---------------------------------------------------------------------------

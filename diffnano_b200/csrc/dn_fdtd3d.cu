@@ -513,6 +513,7 @@ __global__ void __launch_bounds__(Geo64::NCW * 32, 2)
   // ---- march -----------------------------------------------------------------
   for (int i = z0; i < z1; ++i) {
     const bool has_next = (i + 1 < D);
+    if (i == max(z0, z1 - 2)) pdl_release();
     if ((i == 0 && !wait_full(q)) || (has_next && !wait_full(q + 1))) {
       fail();
       return;
@@ -685,11 +686,17 @@ int launch_all(const StepParams<T>& base, const TmapSet& ta, const TmapSet& tb, 
   DN_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)smem));
   StepParams<T> p = base;
+  // Dependent launches: a step's CTAs come up and load their profiles while the last
+  // planes of the step before are marched (2.5 us of each step on B200; released from
+  // its first plane on, a step's CTAs spread unevenly over the SMs behind the running
+  // ones, and 256^3 lost 5 %).
   for (int n = 0; n < nsteps; ++n) {
     const bool even = (n % 2) == 0;
     set_io(&p, even ? fa : fb, even ? fb : fa);
     p.t = t0 + n;
-    kern<<<nctas, nt, smem, s>>>(p, even ? ta : tb, plan, rec);
+    const int rc = launch_chained(kern, (unsigned)nctas, (unsigned)nt, smem, s, n > 0, p,
+                                  even ? ta : tb, plan, rec);
+    if (rc != DN_OK) return rc;
   }
   DN_CUDA_CHECK(cudaGetLastError());
   return DN_OK;

@@ -31,6 +31,26 @@ inline unsigned used_mask(bool is3d, int pol) {
                       : ((1u << DN_HZ) | (1u << DN_EX) | (1u << DN_EY));
 }
 
+// Launch on stream s; `chained`: as a dependent launch of the kernel launched
+// before it on s, which must pass pdl_release() and which this one waits for in
+// pdl_wait() before it touches anything a kernel of the chain writes.
+template <typename K, typename... A>
+int launch_chained(K kern, unsigned blocks, unsigned threads, size_t smem, cudaStream_t s,
+                   bool chained, const A&... args) {
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.gridDim = dim3(blocks);
+  lc.blockDim = dim3(threads);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = s;
+  lc.attrs = at;
+  lc.numAttrs = chained ? 1 : 0;
+  DN_CUDA_CHECK(cudaLaunchKernelEx(&lc, kern, args...));
+  return DN_OK;
+}
+
 template <typename T>
 int build_params(bool is3d, const dn_grid* g, void* const fa[6], void* const fb[6],
                  const void* ce, const dn_cpml* cpml, const dn_source* src,

@@ -41,7 +41,6 @@ constexpr int NCW = Geo32::NCW;      // consumer warps, two rows each
 constexpr int NT = Geo32::NT;        // + one producer warp
 constexpr int BX = Geo32::BX;        // ring box x: k0-4 .. k0+TX+3
 constexpr int BY = Geo32::BY;        // ring box y: j0-1 .. j0+TY
-constexpr int MIN_CHUNK = 8;         // min planes per CTA range
 constexpr uint32_t WAIT_PROBES = 1u << 16;  // bound on mbarrier probes per wait
 constexpr uint32_t SLEEP_NS = 20000;        // suspend-time hint per probe (~1.3 s bound)
 constexpr unsigned FULL_MASK = 0xffffffffu;
@@ -171,18 +170,6 @@ __device__ int pipe_setup(const Smem<T, L>& sm, const Range& R, int D, int H, in
                           const double* const b[3], const double* const c[3],
                           const int* status) {
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
-    sm.flags[0] = skip ? 0 : R.njobs;
-    sm.flags[1] = 0;
-    sm.flags[2] = 0;
-    for (int s = 0; s < L::S; ++s) sm.release[s] = 0;
-    for (int s = 0; s < L::S; ++s) {
-      mbar_init(&sm.full[s], 1);
-      mbar_init(&sm.empty[s], L::G::NCW);
-    }
-    fence_barrier_init();
-  }
   for (int e = tid; e < L::G::TY + 2; e += blockDim.x) {
     const int j = R.j0 - 1 + e;
     const bool ok = j >= 0 && j < H;
@@ -194,6 +181,23 @@ __device__ int pipe_setup(const Smem<T, L>& sm, const Range& R, int D, int H, in
     const bool ok = kx >= 0 && kx < W;
     sm.sbK[e] = ok ? static_cast<T>(b[2][kx]) : T(1);
     sm.sgK[e] = ok ? static_cast<T>(1.0 + c[2][kx]) : T(1);
+  }
+  if (tid == 0) {
+    for (int s = 0; s < L::S; ++s) {
+      mbar_init(&sm.full[s], 1);
+      mbar_init(&sm.empty[s], L::G::NCW);
+    }
+    fence_barrier_init();
+  }
+  // the profiles and the parameters are older than the run's first launch; the
+  // fields and the status are the previous step's
+  pdl_wait();
+  if (tid == 0) {
+    const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
+    sm.flags[0] = skip ? 0 : R.njobs;
+    sm.flags[1] = 0;
+    sm.flags[2] = 0;
+    for (int s = 0; s < L::S; ++s) sm.release[s] = 0;
   }
   __syncthreads();
   return sm.flags[0];
