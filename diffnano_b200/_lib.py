@@ -137,6 +137,13 @@ SIGNATURES = {
                                    ctypes.POINTER(DnMonitor), c_int32, ctypes.POINTER(DnProbe),
                                    ctypes.POINTER(DnCurlRecord), c_int32, c_int32, c_void_p,
                                    c_void_p, ctypes.POINTER(c_int32), c_void_p, c_int64]),
+    "dn_fdtd3d_workspace_bytes": (c_int64, [ctypes.POINTER(DnGrid), ctypes.POINTER(DnSource),
+                                            ctypes.POINTER(DnMonitor), c_int32, c_int32]),
+    "dn_fdtd3d_run_ws": (c_int32, [ctypes.POINTER(DnGrid), _P6, _P6, c_void_p,
+                                   ctypes.POINTER(DnCpml), ctypes.POINTER(DnSource),
+                                   ctypes.POINTER(DnMonitor), c_int32, ctypes.POINTER(DnProbe),
+                                   ctypes.POINTER(DnCurlRecord), c_int32, c_int32, c_void_p,
+                                   c_void_p, ctypes.POINTER(c_int32), c_void_p, c_int64]),
     "dn_fdtd3d_run": (c_int32, [ctypes.POINTER(DnGrid), _P6, _P6, c_void_p,
                                 ctypes.POINTER(DnCpml), ctypes.POINTER(DnSource),
                                 ctypes.POINTER(DnMonitor), c_int32, ctypes.POINTER(DnProbe),

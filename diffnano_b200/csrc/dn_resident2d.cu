@@ -11,14 +11,6 @@ namespace dn {
 namespace res {
 namespace {
 
-template <typename T>
-__global__ void __launch_bounds__(DFT_WARPS * 32)
-    k_sample_dft(const T* smp, long long step_stride, int nsteps, long long ncell,
-                 const double* phase, int nf, double* acc, const int* status) {
-  if (status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;
-  sample_dft<T>(smp, step_stride, nsteps, ncell, phase, nf, acc);
-}
-
 // The work split of a grid, or none (R = 0) when it does not fit on the chip.
 //
 // A step costs what the busiest warp's block costs (rows per warp) plus the

@@ -1,4 +1,4 @@
-// Monitors of the resident 2-D runs: running DFTs from stored samples, and what
+// Monitors of the resident runs: running DFTs from stored samples, and what
 // monitors add to lambda in the reverse sweep.
 #pragma once
 
@@ -62,6 +62,14 @@ __device__ __forceinline__ void sample_dft(const T* __restrict__ smp, long long 
     }
     __syncthreads();
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(DFT_WARPS * 32)
+    k_sample_dft(const T* smp, long long step_stride, int nsteps, long long ncell,
+                 const double* phase, int nf, double* acc, const int* status) {
+  if (status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0) return;
+  sample_dft<T>(smp, step_stride, nsteps, ncell, phase, nf, acc);
 }
 
 // what a monitor adds to lambda before reverse step t: the sum over its

@@ -209,11 +209,11 @@ class Engine:
         L = _lib.lib()
         fa, fb = (self.B, self.A) if self.cur_b else (self.A, self.B)
         out = ctypes.c_int32(0)
-        fn_name = "dn_fdtd3d_run" if self.is3d else "dn_fdtd2d_run_ws"
+        fn_name = "dn_fdtd3d_run_ws" if self.is3d else "dn_fdtd2d_run_ws"
         no_probe = _lib.DnProbe(component=_lib.DN_NONE)
         with torch.cuda.device(self.device):
             stream = torch.cuda.current_stream(self.device).cuda_stream
-            ws = () if self.is3d else self._workspace()
+            ws = self._workspace()
             rc = getattr(L, fn_name)(
                 ctypes.byref(self.grid), self._ptrs(fa), self._ptrs(fb), self.ce.data_ptr(),
                 ctypes.byref(self.cpml), ctypes.byref(self.src), self.mon_arr,
@@ -226,9 +226,10 @@ class Engine:
             self.cur_b = not self.cur_b
 
     def _workspace(self):
-        """(pointer, bytes) of the 2-D runs' workspace, enough for the longest run."""
+        """(pointer, bytes) of the runs' workspace, enough for the longest run."""
         if self._ws is None:
-            n = int(_lib.lib().dn_fdtd2d_workspace_bytes(
+            L = _lib.lib()
+            n = int((L.dn_fdtd3d_workspace_bytes if self.is3d else L.dn_fdtd2d_workspace_bytes)(
                 ctypes.byref(self.grid), ctypes.byref(self.src), self.mon_arr,
                 len(self.monitors), self.n_steps))
             self._ws = torch.empty(max(n, 0), dtype=torch.uint8, device=self.device)

@@ -193,6 +193,17 @@ int32_t dn_fdtd3d_run(const dn_grid* g, void* const fa[6], void* const fb[6], co
                       int32_t t0, int32_t nsteps, int32_t* status, void* stream,
                       int32_t* final_in_b);
 
+/* dn_fdtd3d_run with a workspace: FP32 grids that fit in the shared memory of the
+ * chip (up to about 90^3) with a source in E or none run all steps in one launch.
+ * Same contract as dn_fdtd2d_run_ws and dn_fdtd2d_workspace_bytes. */
+int64_t dn_fdtd3d_workspace_bytes(const dn_grid* g, const dn_source* src, const dn_monitor* mons,
+                                  int32_t n_mon, int32_t nsteps);
+int32_t dn_fdtd3d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
+                         const dn_cpml* cpml, const dn_source* src, const dn_monitor* mons,
+                         int32_t n_mon, const dn_probe* probe, const dn_curl_record* rec,
+                         int32_t t0, int32_t nsteps, int32_t* status, void* stream,
+                         int32_t* final_in_b, void* ws, int64_t ws_bytes);
+
 /* ---- adjoint (reverse) time stepping ------------------------------------
  * Discrete adjoint of the steps above: runs reverse steps t = t_end-1 down
  * to t_end-nsteps.  `la`/`lb` are 6-pointer sets of adjoint fields (the

@@ -45,6 +45,7 @@ def test_one_call_equals_many(cuda, shape, n_mon, dtype):
                      src_box=_setup.source_box_3d(shape, src), src_comp=_lib.DN_EZ,
                      axes=_lib.DN_AXES_PHYSICAL)
         eng.set_eps(eps)
+        eng._ws = torch.empty(0, dtype=torch.uint8, device=cuda)  # launch by launch
         eng.A[..., :W] = fields
         buf = eng.curl_buffer(T)
         rec = eng.curl_record(buf, 0, T)
