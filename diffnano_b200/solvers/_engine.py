@@ -102,14 +102,23 @@ class Engine:
         self.ce = torch.zeros((D, H, self.Wp), **kw)
         self.cur_b = False
 
-        # CPML profiles: axis 0 = z (D), 1 = y (H), 2 = x (W)
-        self.prof = []
-        for a, n in enumerate(self.shape3):
-            if a == 0 and not is3d:
-                self.prof.append(None)
-                continue
-            b, c = _setup.cpml_profile(n, pml_layers, dl, dt)
-            self.prof.append((b.to(device), c.to(device)))
+        # CPML profiles (axis 0 = z (D), 1 = y (H), 2 = x (W); axes of one length share
+        # theirs) and the monitors' phases
+        if len(monitors) > _lib.DN_MAX_MONITORS:
+            raise ValueError(f"at most {_lib.DN_MAX_MONITORS} monitors per solve")
+        self.monitors = list(monitors)
+        for spec in self.monitors:
+            if not 1 <= len(spec.wavelengths) <= _lib.DN_MAX_FREQS:
+                raise ValueError(f"a monitor takes 1..{_lib.DN_MAX_FREQS} wavelengths")
+        lengths = sorted(set(self.shape3 if is3d else self.shape3[1:]))
+        tables = [t for n in lengths for t in _setup.cpml_profile(n, pml_layers, dl, dt)]
+        tables += [_setup.dft_phase_table(self.n_steps, self.dt, spec.wavelengths)
+                   for spec in self.monitors]
+        tables = _setup.upload_tables(tables, device)
+        prof = {n: (tables[2 * i], tables[2 * i + 1]) for i, n in enumerate(lengths)}
+        self.prof = [None if a == 0 and not is3d else prof[n]
+                     for a, n in enumerate(self.shape3)]
+        self.phases = tables[2 * len(lengths):]
         self.cpml = _lib.DnCpml()
         for a in range(3):
             if self.prof[a] is not None:
@@ -130,17 +139,11 @@ class Engine:
             self.src.n_t = self.wave.numel()
 
         # monitors
-        if len(monitors) > _lib.DN_MAX_MONITORS:
-            raise ValueError(f"at most {_lib.DN_MAX_MONITORS} monitors per solve")
-        self.monitors = list(monitors)
-        self.phases, self.accs = [], []
+        self.accs = []
         self.mon_arr = (_lib.DnMonitor * max(1, len(self.monitors)))()
         for m, spec in enumerate(self.monitors):
-            if not 1 <= len(spec.wavelengths) <= _lib.DN_MAX_FREQS:
-                raise ValueError(f"a monitor takes 1..{_lib.DN_MAX_FREQS} wavelengths")
-            ph = _setup.dft_phase_table(self.n_steps, self.dt, spec.wavelengths).to(device)
+            ph = self.phases[m]
             acc = torch.zeros((len(spec.wavelengths), spec.cells, 2), dtype=F64, device=device)
-            self.phases.append(ph)
             self.accs.append(acc)
             M = self.mon_arr[m]
             M.component = spec.component

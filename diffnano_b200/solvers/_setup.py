@@ -27,16 +27,29 @@ def cpml_profile(size: int, pml_layers: int, dl: float, dt: float,
     sigma_s = sigma*dl/dt, alpha = 0.02 sigma_s, b = exp(-(sigma_s+alpha) dt),
     c = sigma_s (b-1)/(sigma_s+alpha+1e-30) where sigma_s+alpha > 1e-30, else 0.
     """
-    sigma = torch.zeros(size, dtype=F64)
+    sigma = [0.0] * size
     for i in range(max(0, pml_layers)):
         val = sigma_max * ((pml_layers - i) / pml_layers) ** order
         sigma[i] = val
         sigma[size - 1 - i] = val
-    s = sigma * dl / dt
+    s = torch.tensor(sigma, dtype=F64) * dl / dt
     a = 0.02 * s
     b = torch.exp(-(s + a) * dt)
     c = torch.where(s + a > 1e-30, s * (b - 1.0) / (s + a + 1e-30), torch.zeros_like(s))
     return b, c
+
+
+def upload_tables(tables, device) -> list:
+    """FP64 CPU tensors as device tensors, in one copy (16-byte aligned views of one
+    buffer)."""
+    sizes = [(t.numel() + 1) // 2 * 2 for t in tables]
+    host = torch.zeros(sum(sizes), dtype=F64)
+    at = 0
+    for t, n in zip(tables, sizes):
+        host[at:at + t.numel()] = t.reshape(-1)
+        at += n
+    dev = host.to(device)
+    return [v[:t.numel()].view(t.shape) for v, t in zip(dev.split(sizes), tables)]
 
 
 def waveform_table(n_steps: int, dt: float, omega: float, source: dict) -> torch.Tensor:
