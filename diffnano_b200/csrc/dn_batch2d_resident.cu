@@ -1,6 +1,7 @@
 // Batched TM runs and reverse sweeps on the chip (dn_resident2d.cuh, struct
 // List): which CTA takes which bands of which grids, and the entry points.
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <numeric>
 #include <vector>
@@ -42,6 +43,31 @@ struct Plan {
 
 inline long long up16(long long x) { return (x + 15) / 16 * 16; }
 
+// us per step of bands with R = 1, 2, 4 rows per warp (B200, FP32, 16 warps): run,
+// recorded run, reverse sweep
+constexpr double STEP_US[3][3] = {{0.79, 1.04, 1.82}, {0.95, 1.35, 4.0}, {2.0, 3.1, 0.0}};
+
+// The CTAs by the steps they have been given, fewest first.
+struct Loads {
+  std::vector<std::pair<double, int>> v;
+  explicit Loads(int n_cta) : v(n_cta) {
+    for (int c = 0; c < n_cta; ++c) v[c] = {0.0, c};
+  }
+  // the next grid: its bands go to the CTAs that are free first, all of which are
+  // then busy until it ends; give(band, cta)
+  template <typename F>
+  void add(int bands, int steps, const F& give) {
+    const double end = v[bands - 1].first + steps;
+    for (int b = 0; b < bands; ++b) {
+      give(b, v[b].second);
+      v[b].first = end;
+    }
+    const auto rest = v.begin() + bands;
+    std::rotate(v.begin(), rest,
+                std::upper_bound(rest, v.end(), std::pair<double, int>(end, INT_MAX)));
+  }
+};
+
 // false: some grid does not fit, or the batch is not a TM one
 bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint, Plan* P) {
   const long long off = batch2d_inst_offset(cfg, insts);
@@ -63,20 +89,29 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
     G.bands = G.groups ? (I.H + G.groups * R - 1) / (G.groups * R) : 0;
     return G;
   };
-  // the fewest rows per warp for which every band has a CTA of its own, else the
-  // most that registers hold: fewer bands, less time in exchanges per cell
-  // (256^2 FP32 x 96: R = 4 20 ms, R = 2 24 ms)
-  const int r_last = adjoint ? 2 : 4;
-  int R = 1;
-  for (;; R *= 2) {
-    long long bands = 0;
-    for (int b = 0; b < n; ++b) {
-      const ListGrid G = grid_of(insts[b], R);
-      if (G.groups == 0) return false;
-      bands += G.bands;
+  // The rows per warp with which the last CTA is done first: more rows are fewer and
+  // slower turns (96 x 256^2, 2000 steps: 38 / 23 / 22 ms with R = 1 / 2 / 4; 12
+  // recorded grids of 100^2 to 512^2: 3.8 / 2.8 / 3.9 ms, and their sweep 7.8 / 6.5)
+  bool record = false;
+  for (int b = 0; b < n; ++b) record = record || insts[b].curl != nullptr;
+  int R = 0;
+  double best = 0.0;
+  for (int r = 1; r <= (adjoint ? 2 : 4); r *= 2) {
+    Loads loads(nsm);
+    bool fits = true;
+    for (int k = 0; k < n && fits; ++k) {
+      const ListGrid G = grid_of(insts[order[k]], r);
+      fits = G.groups > 0 && G.bands <= nsm;
+      if (fits) loads.add(G.bands, insts[order[k]].n_steps, [](int, int) {});
     }
-    if (bands <= nsm || R == r_last) break;
+    if (!fits) continue;
+    const double t = loads.v.back().first * STEP_US[adjoint ? 2 : record ? 1 : 0][r / 2];
+    if (R == 0 || t < best) {
+      best = t;
+      R = r;
+    }
   }
+  if (R == 0) return false;
   Head& h = P->h;
   h.n_inst = n;
   h.n_cta = nsm;
@@ -89,14 +124,11 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
     Group g{};
     g.first = k;
     long long mail = 0, sample = 0;
-    // each grid's bands go to the CTAs that are free first
-    std::vector<double> load(nsm, 0.0);
+    Loads loads(nsm);
     std::vector<std::vector<ListJob>> lists(nsm);
-    std::vector<int> by(nsm);
     for (; k < n; ++k) {
       const dn_batch2d_inst& I = insts[order[k]];
       ListGrid G = grid_of(I, R);
-      if (G.bands > nsm) return false;
       long long cells = 0, bytes = 0;
       if (I.mon_comp != DN_NONE) {
         cells = (long long)(I.mon_box.hi[1] - I.mon_box.lo[1]) *
@@ -112,13 +144,7 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
       sample += bytes;
       g.max_cells = std::max(g.max_cells, cells);
       P->grids.push_back(G);
-      std::iota(by.begin(), by.end(), 0);
-      std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return load[a] < load[b]; });
-      const double end = load[by[G.bands - 1]] + I.n_steps;
-      for (int b = 0; b < G.bands; ++b) {
-        lists[by[b]].push_back({k, b});
-        load[by[b]] = end;
-      }
+      loads.add(G.bands, I.n_steps, [&](int b, int cta) { lists[cta].push_back({k, b}); });
     }
     g.count = k - g.first;
     g.mail_words = mail;
