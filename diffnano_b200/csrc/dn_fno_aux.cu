@@ -133,7 +133,9 @@ __global__ void k_readout(const unsigned short* __restrict__ x, const float* __r
 }
 
 // the same with four consecutive columns w per thread (W % 4 == 0, x 8-byte
-// aligned): 8-byte loads, a warp reads 256 contiguous bytes per row h
+// aligned): 8-byte loads, a warp reads 256 contiguous bytes per row h; 16 rows are
+// loaded before they are added (bound by loads in flight: batch 128, 64 channels,
+// 128^2 on B200 128 -> 49 us)
 __global__ void k_readout4(const unsigned short* __restrict__ x, const float* __restrict__ r,
                            long long nb, int H, int W, int C, unsigned short* __restrict__ out) {
   const int W4 = W / 4;
@@ -145,15 +147,23 @@ __global__ void k_readout4(const unsigned short* __restrict__ x, const float* __
     const long long b = i / ((long long)W4 * C);
     const unsigned short* xp = x + (b * C + c) * (long long)H * W + w0;
     float s0 = 0.0f, s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
-#pragma unroll 4
-    for (int h = 0; h < H; ++h) {
-      const uint2 u = *reinterpret_cast<const uint2*>(xp + (long long)h * W);
-      const float rv = r[h * C + c];
+    auto add = [&](const uint2 u, float rv) {
       s0 = fmaf(rv, __uint_as_float(u.x << 16), s0);
       s1 = fmaf(rv, __uint_as_float(u.x & 0xFFFF0000u), s1);
       s2 = fmaf(rv, __uint_as_float(u.y << 16), s2);
       s3 = fmaf(rv, __uint_as_float(u.y & 0xFFFF0000u), s3);
+    };
+    int h = 0;
+    for (; h + 16 <= H; h += 16) {
+      uint2 u[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q)
+        u[q] = __ldcs(reinterpret_cast<const uint2*>(xp + (long long)(h + q) * W));
+#pragma unroll
+      for (int q = 0; q < 16; ++q) add(u[q], __ldg(r + (h + q) * C + c));
     }
+    for (; h < H; ++h)
+      add(*reinterpret_cast<const uint2*>(xp + (long long)h * W), __ldg(r + h * C + c));
     unsigned short* o = out + (b * W + w0) * C + c;
     o[0] = f2bf(s0);
     o[C] = f2bf(s1);
