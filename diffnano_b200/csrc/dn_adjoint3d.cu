@@ -217,6 +217,19 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     ++q;
   }
 
+  // The FP64 gradient of the owned cells; FP32: loaded one plane ahead, since within
+  // the plane its latency is longer than the work on lH' (B200, 96 x 192 x 192: 63 ->
+  // 60 us per step; FP64 has no registers left for it).
+  constexpr bool AHEAD = sizeof(T) == 4;
+  double gnext[2];
+  auto load_grad = [&](int i) {
+    const long long o = i * pz + (long long)ja * py + k;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      gnext[r] = i < z1 && ja + r < H && kin ? p.grad[o + r * py] : 0.0;
+  };
+  if (AHEAD) load_grad(z0);
+
   // ---- march -----------------------------------------------------------------
   for (int i = z0; i < z1; ++i) {
     const bool has_next = (i + 1 < D);
@@ -232,12 +245,10 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     const T fi_next = has_next ? T(1) : T(0);
     const T* cur = sm.arr(q, 0) + 2 * w * BX + lane + 4;
     const T* nxt = has_next ? sm.arr(q + 1, 0) + 2 * w * BX + lane + 4 : cur;
-    // issue the FP64 gradient loads now; they are consumed after lH'
     const long long o_plane = i * pz + (long long)ja * py + k;
-    double gpre[2];
-#pragma unroll
-    for (int r = 1; r < 3; ++r)
-      gpre[r - 1] = (ja + r - 1 < H && kin) ? p.grad[o_plane + (r - 1) * py] : 0.0;
+    if (!AHEAD) load_grad(i);
+    const double gpre[2] = {gnext[0], gnext[1]};
+    if (AHEAD) load_grad(i + 1);
 
     // ---- lH' of rows ja-1, ja, ja+1 --------------------------------------
     T LHx[3], LHy[3], LHz[3];
