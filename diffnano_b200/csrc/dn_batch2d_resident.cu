@@ -45,7 +45,7 @@ inline long long up16(long long x) { return (x + 15) / 16 * 16; }
 
 // us per step of bands with R = 1, 2, 4 rows per warp (B200, FP32, 16 warps): run,
 // recorded run, reverse sweep
-constexpr double STEP_US[3][3] = {{0.79, 1.04, 1.82}, {0.95, 1.35, 4.0}, {2.0, 3.1, 0.0}};
+constexpr double STEP_US[3][3] = {{0.79, 1.04, 1.82}, {0.95, 1.35, 4.0}, {1.4, 2.6, 0.0}};
 
 // The CTAs by the steps they have been given, fewest first.
 struct Loads {
@@ -91,7 +91,7 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
   };
   // The rows per warp with which the last CTA is done first: more rows are fewer and
   // slower turns (96 x 256^2, 2000 steps: 38 / 23 / 22 ms with R = 1 / 2 / 4; 12
-  // recorded grids of 100^2 to 512^2: 3.8 / 2.8 / 3.9 ms, and their sweep 7.8 / 6.5)
+  // recorded grids of 100^2 to 512^2: 3.8 / 2.8 / 3.9 ms)
   bool record = false;
   for (int b = 0; b < n; ++b) record = record || insts[b].curl != nullptr;
   int R = 0;

@@ -5,13 +5,13 @@
 // lambda_Hy of the row above and lambda_Hx of the column to the left are copies
 // that the warp updates itself.  The FP64 gradient of the block's cells stays in
 // registers for the whole sweep (it was a read and a write of 8 bytes per cell and
-// step), the step's curl row is loaded one step ahead, and what the monitors add
+// step), its sum is taken while the rows are on their way, and what the monitors add
 // to lambda_Ez before a step comes as a table, computed for all steps at once.
 //
 // Bound by the same chain as the forward run (row received, block updated, row
 // sent).  Measured on B200, 300 x 413 FP32, one monitor row at three wavelengths:
-// 1.9 us per reverse step; before, two launches per step (injection 2.2 us and
-// reverse step 5.2 us, and the gaps between them).
+// 1.5 us per reverse step (1.2 without a monitor); before, two launches per step
+// (injection 2.2 us and reverse step 5.2 us, and the gaps between them).
 #pragma once
 
 #include "dn_resident2d_dev.cuh"
@@ -81,12 +81,44 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
         adds[m].hi[1] > j0)
       add_mask |= 1u << m;
 
+  // The block's first monitor, when it adds to one row of the block in 16-byte pieces,
+  // is read a step ahead into registers (read when it is added, it cost every step of
+  // the grid 0.4 us).
+  V pre{};
+  int pre_m = -1;  // its index
+  auto pre_row = [&](const Samples<T>& M) { return M.lo[0] > ia ? M.lo[0] - ia : 0; };
+  auto fetch_add = [&](int n) {
+    const Samples<T>& M = adds[pre_m];
+    const long long row = (ia + pre_row(M) - M.lo[0]) * (long long)(M.hi[1] - M.lo[1]);
+    ld16_where<T>(M.buf + n * M.step_stride + row + (jv - M.lo[1]),
+                  n + 1 < J.nsteps && jv >= M.lo[1] && jv < M.hi[1], pre);
+  };
+  if (add_mask) {
+    const Samples<T>& M = adds[__ffs(add_mask) - 1];
+    const int hi = M.hi[0] < ia + R ? M.hi[0] - ia : R;
+    // rows of the table on 16-byte boundaries (a step's are a multiple long)
+    if (hi - pre_row(M) == 1 && M.lo[1] % VEC == 0 &&
+        (M.hi[0] - M.lo[0] == 1 || (M.hi[1] - M.lo[1]) % VEC == 0)) {
+      pre_m = __ffs(add_mask) - 1;
+      add_mask &= add_mask - 1;
+      fetch_add(0);
+    }
+  }
+
   auto coef_e = [&](int r) -> V { return CES ? ld16<T>(ces + r * 512) : ce[CES ? 0 : r]; };
-  auto step = [&](int par, int n) {
-    const T* const fl = K.l_edge + par * B::EDGE_P;
-    const T* const fr = K.r_edge + par * B::EDGE_P;
-    const V bx = ld16<T>(K.cc), hk = ld16<T>(K.cc + CARR);
-    const V gk = ld16<T>(K.cc + 2 * CARR);
+  // Curl rows come from memory into L2 two steps before they are loaded, and into
+  // registers one step before they are used (300 x 413, us per step: 1.67 when the
+  // load was waited for on the spot, 1.31 without, 1.22 with the rows in L2 too).
+  constexpr int CURL_AHEAD = 2;
+  auto fetch_curl = [&](int n) {
+    if (n >= J.nsteps || !live || !any) return;
+    const T* const from = J.curl - (long long)n * J.curl_stride + o0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (ia + r < H) asm volatile("prefetch.global.L2 [%0];" ::"l"(from + r * py));
+  };
+  // the gradient's share of step n, and the curl of the step after it
+  auto gradient = [&](int n) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
 #pragma unroll
@@ -96,8 +128,16 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
     if (n + 1 < J.nsteps) {
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        c[r] = K.load(J.curl - (long long)(n + 1) * J.curl_stride, o0 + r * py, ia + r < H, W);
+        ld16_where<T>(J.curl - (long long)(n + 1) * J.curl_stride + o0 + r * py,
+                      live && any && ia + r < H, c[r]);
     }
+    fetch_curl(n + 1 + CURL_AHEAD);
+  };
+  auto step = [&](int par) {
+    const T* const fl = K.l_edge + par * B::EDGE_P;
+    const T* const fr = K.r_edge + par * B::EDGE_P;
+    const V bx = ld16<T>(K.cc), hk = ld16<T>(K.cc + CARR);
+    const V gk = ld16<T>(K.cc + 2 * CARR);
     // lambda_Hy' of row ia-1 and its vy
     V vy_up;
     {
@@ -139,14 +179,31 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
     }
   };
 
+  for (int n = 1; n <= CURL_AHEAD; ++n) fetch_curl(n);
+  gradient(0);
   K.publish(0, u);
   __syncthreads();  // also: the coefficients are in place
 
   auto advance = [&](auto par_c, int n) -> bool {
     constexpr int PAR = decltype(par_c)::value;
     constexpr int NXT = PAR ^ 1;
-    if (K.active) step(PAR, n);
+    if (K.active) step(PAR);
     if (n + 1 == J.nsteps) return false;
+    if (pre_m >= 0) {
+      const Samples<T>& M = adds[pre_m];
+      const int pr = pre_row(M), left = jv >= M.lo[1] ? M.hi[1] - jv : 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        if (r != pr) continue;
+        if (left >= VEC) {
+          e[r] = addv<T>(e[r], pre);
+        } else {
+#pragma unroll
+          for (int q = 0; q < VEC; ++q)
+            if (q < left) e[r].set(q, e[r].get(q) + pre.get(q));
+        }
+      }
+    }
     if (add_mask) {
 #pragma unroll 1
       for (int m = 0; m < n_add; ++m) {
@@ -176,6 +233,8 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
       K.publish(NXT, u);
     }
     __syncthreads();
+    if (K.active) gradient(n + 1);  // while the rows are on their way
+    if (pre_m >= 0) fetch_add(n + 1);
     const bool go = K.gather(NXT, n, u_up, u_dn);
     if (ia <= 1) {  // row ia-1 = 0 has no weight on its own u; row -1 does not exist
 #pragma unroll

@@ -286,6 +286,20 @@ __device__ __forceinline__ void st16(unsigned char* a, const Pack<T>& v) {
   *reinterpret_cast<ulonglong2*>(a) = make_ulonglong2(bits(v.p[0]), bits(v.p[1]));
 }
 
+// the 16 bytes at `a` where ok, else v as it was: one predicated load straight into
+// v's registers.  (A choice between the value read and another one is made on the
+// spot: it waits for the load that was meant to be under way.)
+template <typename T>
+__device__ __forceinline__ void ld16_where(const T* a, bool ok, Pack<T>& v) {
+  uint64_t x = bits(v.p[0]), y = bits(v.p[1]);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p ld.global.v2.b64 {%0, %1}, [%2];\n\t}"
+      : "+l"(x), "+l"(y)
+      : "l"(a), "r"((int)ok));
+  from_bits(x, v.p[0]);
+  from_bits(y, v.p[1]);
+}
+
 // bounded wait for a phase of an mbarrier
 __device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity) {
   for (unsigned n = 0; n < PROBE_LIMIT; ++n)

@@ -169,23 +169,17 @@ def _sweep(eng, ws, la, lb, rec, grad, mon_arr, n_mon, t_end, T):
     return lb if out.value else la
 
 
-@pytest.mark.gpu
-@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
-@pytest.mark.parametrize("H,W", [s for s in SHAPES if s[0] * s[1] < 500_000])
-def test_reverse_sweep(cuda, H, W, dtype):
-    """From random adjoint fields, curl terms and a running gradient, with a row
-    and a box monitor whose gradients enter before every step."""
-    f = _lib.DN_EZ
-    mons = [MonitorSpec("row", f, ((0, 1), (H // 2, H // 2 + 1), (0, W)), [1500.0, 1600.0]),
-            MonitorSpec("box", f, ((0, 1), (0, (H + 1) // 2), (W // 2, W)), [1550.0])]
+def _compare_sweeps(cuda, H, W, dtype, mons):
+    """From random adjoint fields, curl terms and a running gradient, with monitors
+    whose gradients enter before every step."""
     for T in (9, 24):
         eng = _engine(H, W, _lib.DN_TM, dtype, T + 3, mons)
         g = torch.Generator().manual_seed(T)
         rand = lambda *s: torch.randn(*s, dtype=torch.float64, generator=g)  # noqa: E731
         lam, curl, grad0 = rand(6, 1, H, W), rand(T, H, W), rand(1, H, W)
         gm = [rand(*a.shape).to(cuda) for a in eng.accs]
-        mon_arr = (_lib.DnMonitor * 2)()
-        for m in range(2):
+        mon_arr = (_lib.DnMonitor * len(mons))()
+        for m in range(len(mons)):
             ctypes.memmove(ctypes.byref(mon_arr[m]), ctypes.byref(eng.mon_arr[m]),
                            ctypes.sizeof(_lib.DnMonitor))
             mon_arr[m].acc = gm[m].data_ptr()
@@ -198,7 +192,33 @@ def test_reverse_sweep(cuda, H, W, dtype):
             la[..., :W] = lam.to(cuda, dtype)
             grad = torch.zeros(1, H, eng.Wp, dtype=torch.float64, device=cuda)
             grad[..., :W] = grad0.to(cuda)
-            out = _sweep(eng, ws, la, lb, rec, grad, mon_arr, 2, T + 2, T)
+            out = _sweep(eng, ws, la, lb, rec, grad, mon_arr, len(mons), T + 2, T)
             got.append([out[c, ..., :W].clone() for c in _comps(_lib.DN_TM)] + [grad[..., :W]])
         for a, b in zip(*got):
             assert rel_l2(a, b) < 2 * _tol(dtype, T)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("H,W", [s for s in SHAPES if s[0] * s[1] < 500_000])
+def test_reverse_sweep(cuda, H, W, dtype):
+    f = _lib.DN_EZ
+    _compare_sweeps(cuda, H, W, dtype, [
+        MonitorSpec("row", f, ((0, 1), (H // 2, H // 2 + 1), (0, W)), [1500.0, 1600.0]),
+        MonitorSpec("box", f, ((0, 1), (0, (H + 1) // 2), (W // 2, W)), [1550.0])])
+
+
+# what a block reads a step ahead and what it does not: rows that end inside a lane's
+# columns, rows of a wider table, two of a block's rows, columns off the 16 bytes; two
+# monitors on the same cells, the one read ahead first or second
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("boxes", [[((50, 51), (8, 61))], [((40, 45), (4, 132))],
+                                   [((40, 45), (4, 131))], [((70, 71), (3, 140))],
+                                   [((60, 61), (0, 141)), ((58, 63), (2, 99))],
+                                   [((58, 63), (2, 99)), ((60, 61), (0, 141))],
+                                   [((96, 97), (136, 141)), ((96, 97), (136, 141))]])
+@pytest.mark.parametrize("H", [97, 390])
+def test_reverse_sweep_monitors(cuda, H, boxes, dtype):
+    _compare_sweeps(cuda, H, 141, dtype, [
+        MonitorSpec(str(n), _lib.DN_EZ, ((0, 1), *b), [1550.0]) for n, b in enumerate(boxes)])
