@@ -204,8 +204,9 @@ __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int ba
       if (has_ghosts) ghosts();
       K.post(NXT, n, f);
       if (K.active) K.publish(NXT, f);
+      __syncthreads();
     }
-    if (SMP && smp_mask) {
+    if (SMP && smp_mask) {  // (while the rows are on their way)
 #pragma unroll 1
       for (int m = 0; m < n_smp; ++m) {
         if (!((smp_mask >> m) & 1u)) continue;
@@ -232,7 +233,6 @@ __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int ba
       }
     }
     if (!more) return false;
-    __syncthreads();
     return K.gather(NXT, n, f_up, f_dn);
   };
   using P0 = std::integral_constant<int, 0>;
