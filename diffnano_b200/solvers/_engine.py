@@ -166,7 +166,7 @@ class Engine:
             self.probe.n_t = self.probe_out.numel()
 
         self.status = torch.zeros(1, dtype=torch.int32, device=device)
-        self._ws = None  # 2-D: workspace of the resident runs, made by the first run
+        self._ws = None  # workspace of the resident runs, made by the first run
 
     # ------------------------------------------------------------------
     def set_eps(self, eps: torch.Tensor) -> None:
@@ -235,7 +235,10 @@ class Engine:
             n = int((L.dn_fdtd3d_workspace_bytes if self.is3d else L.dn_fdtd2d_workspace_bytes)(
                 ctypes.byref(self.grid), ctypes.byref(self.src), self.mon_arr,
                 len(self.monitors), self.n_steps))
-            self._ws = torch.empty(max(n, 0), dtype=torch.uint8, device=self.device)
+            try:
+                self._ws = torch.empty(max(n, 0), dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:  # without one the steps go launch by launch
+                self._ws = torch.empty(0, dtype=torch.uint8, device=self.device)
         return self._ws.data_ptr() if self._ws.numel() else None, self._ws.numel()
 
     # ------------------------------------------------------------------

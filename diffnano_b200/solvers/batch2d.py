@@ -278,7 +278,10 @@ class FDTDBatch2D:
                 self._plans[adjoint] = (host, dev, int(ws.value))
         need = max((p[2] for p in self._plans.values()), default=0)
         if self._ws is None or self._ws.numel() < need:
-            self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            try:
+                self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:  # the persistent kernel needs none
+                self._ws, self._plans = None, {}
 
     def uses_resident(self, fwd: bool, grad: bool) -> bool:
         """Whether a forward (with or without gradient) or backward run keeps the
