@@ -44,33 +44,33 @@ struct AdjCfg {
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
 __device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
 
+// The monitors' gradients of step t - 1 added to the fields that this thread has
+// stored (rows ja, ja + 1 of column k, planes z0 .. z1 - 1), in monitor order.  After
+// the march: a launch of its own per monitor and step took 3.3 us and a launch gap, and
+// the same adds beside the stores cost the march registers (reference axes, us per step
+// with a launch / beside the stores / here: 192^3 113 / 124 / 104, 256^3 260 / 301 / 247).
 template <typename T>
-__device__ __forceinline__ bool any_monitor(const AdjParams<T>& p, int i) {
-  bool any = false;
-#pragma unroll
-  for (int m = 0; m < DN_MAX_MONITORS; ++m) any |= m < p.n_mon && p.mon[m].box.has_plane(i);
-  return any;
-}
-
-// The monitors' gradients of step t - 1 on one cell's stored fields, in monitor
-// order (a launch of its own per monitor and step took 3.3 us and a launch gap).
-template <typename T>
-__device__ __forceinline__ void inject_cell(const AdjParams<T>& p, int i, int j, int k, T& ex, T& ey,
-                                            T& ez, T& hx, T& hy, T& hz) {
+__device__ __forceinline__ void inject_monitors_after(const AdjParams<T>& p, int z0, int z1,
+                                                      int ja, int k) {
 #pragma unroll
   for (int m = 0; m < DN_MAX_MONITORS; ++m) {
     if (m >= p.n_mon) break;
     const MonDev& M = p.mon[m];
-    if (!M.box.contains(i, j, k)) continue;
-    const T g = static_cast<T>(
-        monitor_grad(M, M.phase + (long long)(p.t - 1) * M.nf * 2, M.box.offset(i, j, k)));
+    if (k < M.box.lo[2] || k >= M.box.hi[2]) continue;
     const int c = M.comp;
-    ex = c == DN_EX ? add_rn(ex, g) : ex;
-    ey = c == DN_EY ? add_rn(ey, g) : ey;
-    ez = c == DN_EZ ? add_rn(ez, g) : ez;
-    hx = c == DN_HX ? add_rn(hx, g) : hx;
-    hy = c == DN_HY ? add_rn(hy, g) : hy;
-    hz = c == DN_HZ ? add_rn(hz, g) : hz;
+    T* const lam = c == DN_EX   ? p.out[DN_EX]
+                   : c == DN_EY ? p.out[DN_EY]
+                   : c == DN_EZ ? p.out[DN_EZ]
+                   : c == DN_HX ? p.out[DN_HX]
+                   : c == DN_HY ? p.out[DN_HY]
+                                : p.out[DN_HZ];
+    const double* const ph = M.phase + (long long)(p.t - 1) * M.nf * 2;
+    const int i0 = max(z0, M.box.lo[0]), i1 = min(z1, M.box.hi[0]);
+    for (int i = i0; i < i1; ++i)
+      for (int j = max(ja, M.box.lo[1]); j < min(ja + 2, M.box.hi[1]); ++j) {
+        const long long o = i * p.pz + j * p.py + k;
+        lam[o] = add_rn(lam[o], static_cast<T>(monitor_grad(M, ph, M.box.offset(i, j, k))));
+      }
   }
 }
 
@@ -217,10 +217,11 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     ++q;
   }
 
-  // The FP64 gradient of the owned cells; FP32: loaded one plane ahead, since within
-  // the plane its latency is longer than the work on lH' (B200, 96 x 192 x 192: 63 ->
-  // 60 us per step; FP64 has no registers left for it).
-  constexpr bool AHEAD = sizeof(T) == 4;
+  // The FP64 gradient of the owned cells; FP32 with physical axes: loaded one plane
+  // ahead, since within the plane its latency is longer than the work on lH' (B200, us
+  // per step: 192^3 107 -> 103, 256^3 258 -> 241).  The others have no registers left
+  // for it (reference axes 256^3: 247 -> 318).
+  constexpr bool AHEAD = sizeof(T) == 4 && AXES == DN_AXES_PHYSICAL;
   double gnext[2];
   auto load_grad = [&](int i) {
     const long long o = i * pz + (long long)ja * py + k;
@@ -288,7 +289,6 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     const T hvyk0 = __shfl_sync(FULL_MASK, hvyk, 0), hvyk1 = __shfl_sync(FULL_MASK, hvyk, 1);
     const T hvzk0 = __shfl_sync(FULL_MASK, hvzk, 0), hvzk1 = __shfl_sync(FULL_MASK, hvzk, 1);
 
-    const bool special = any_monitor(p, i);
     // ---- previous adjoint fields of rows ja, ja+1 ---------------------------
     const T* ct = sm.tile_arr(q, NRING_A, 0) + (2 * w) * TX + lane;
     constexpr int TE = L::TILE_ARR / (int)sizeof(T);
@@ -315,23 +315,21 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
         const T ex_b = AXES == DN_AXES_REFERENCE ? bJ[r] * bK : bJ[r] * bI;
         const T ey_b = AXES == DN_AXES_REFERENCE ? bK * bJ[r] : bI * bK;
         const T ez_b = bK * bJ[r];
-        T nlex = ex_b * lex + (vyi - pvyi[r - 1]) - (vzj - vzj_m);
-        T nley = ey_b * ley - (vxi - pvxi[r - 1]) + (vzk - vzk_m);
-        T nlez = ez_b * lez + (vxj - vxj_m) - (vyk - vyk_m);
+        const T nlex = ex_b * lex + (vyi - pvyi[r - 1]) - (vzj - vzj_m);
+        const T nley = ey_b * ley - (vxi - pvxi[r - 1]) + (vzk - vzk_m);
+        const T nlez = ez_b * lez + (vxj - vxj_m) - (vyk - vyk_m);
         const long long o = o_plane + (r - 1) * py;
         const int et = (r - 1) * TX;
         const double gsum = static_cast<double>(lex) * static_cast<double>(ct[et]) +
                             static_cast<double>(ley) * static_cast<double>(ct[TE + et]) +
                             static_cast<double>(lez) * static_cast<double>(ct[2 * TE + et]);
         p.grad[o] = gpre[r - 1] + gsum;
-        T nlhx = bJ[r] * LHx[r], nlhy = hy_b * LHy[r], nlhz = bK * LHz[r];
-        if (special) inject_cell(p, i, j, k, nlex, nley, nlez, nlhx, nlhy, nlhz);
         p.out[DN_EX][o] = nlex;
         p.out[DN_EY][o] = nley;
         p.out[DN_EZ][o] = nlez;
-        p.out[DN_HX][o] = nlhx;
-        p.out[DN_HY][o] = nlhy;
-        p.out[DN_HZ][o] = nlhz;
+        p.out[DN_HX][o] = bJ[r] * LHx[r];
+        p.out[DN_HY][o] = hy_b * LHy[r];
+        p.out[DN_HZ][o] = bK * LHz[r];
       }
       pvxi[r - 1] = vxi;
       pvyi[r - 1] = vyi;
@@ -340,6 +338,7 @@ __global__ void __launch_bounds__(NT, AdjCfg<T>::MINB)
     ++q;
   }
   if (z1 < D) release(q);
+  if (p.n_mon > 0 && kin) inject_monitors_after(p, z0, z1, ja, k);
 }
 
 template <typename T, int AXES>
@@ -381,7 +380,7 @@ int launch_adj(AdjParams<T> p, void* const la[6], void* const lb[6], const dn_gr
       p.out[c] = static_cast<T*>(even ? lb[c] : la[c]);
     }
     // the first step's monitor gradients go in ahead of it, those of each further
-    // one with the stores of the step before
+    // one at the end of the step before
     p.t = t_end - 1 - n;
     if (n == 0 && n_mon > 0 && (rc = inject_monitors<T>(p, mons, n_mon, true, 0, s)) != DN_OK)
       return rc;

@@ -689,13 +689,15 @@ int launch_all(const StepParams<T>& base, const TmapSet& ta, const TmapSet& tb, 
   // Dependent launches: a step's CTAs come up and load their profiles while the last
   // planes of the step before are marched (2.5 us of each step on B200; released from
   // its first plane on, a step's CTAs spread unevenly over the SMs behind the running
-  // ones, and 256^3 lost 5 %).
+  // ones, and 256^3 lost 5 %).  Steps that write a curl record on large grids do without:
+  // 192^3 99 -> 95 us per step with them, 256^3 206 -> 213.
+  const bool chain = !REC || (long long)base.D * base.H * base.W <= 1LL << 23;
   for (int n = 0; n < nsteps; ++n) {
     const bool even = (n % 2) == 0;
     set_io(&p, even ? fa : fb, even ? fb : fa);
     p.t = t0 + n;
-    const int rc = launch_chained(kern, (unsigned)nctas, (unsigned)nt, smem, s, n > 0, p,
-                                  even ? ta : tb, plan, rec);
+    const int rc = launch_chained(kern, (unsigned)nctas, (unsigned)nt, smem, s, chain && n > 0,
+                                  p, even ? ta : tb, plan, rec);
     if (rc != DN_OK) return rc;
   }
   DN_CUDA_CHECK(cudaGetLastError());
