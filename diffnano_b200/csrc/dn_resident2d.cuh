@@ -27,7 +27,7 @@
 // row received -> block updated -> row sent -> received by the neighbour, and
 // the issue slots of the busiest warp.  Measured on B200, FP32 TM, us per step
 // (before: the cluster kernel of dn_batch2d.cu, or one launch per step): 100^2
-// 0.42 (2.17), 256^2 with a monitor row 0.93 (3.74), 512^2 0.95 (7.0), 1024^2
+// 0.42 (2.17), 256^2 with a monitor row 0.89 (3.74), 512^2 0.95 (7.0), 1024^2
 // with a monitor row 2.2 (10.4).  What was learned on the way: FP64 monitor
 // sums inside the march cost every step 0.35 - 0.9 us (all bands wait for the
 // band that has them), stored samples 0.02 - 0.15; 255 registers and 8 rows per
