@@ -45,7 +45,7 @@ inline long long up16(long long x) { return (x + 15) / 16 * 16; }
 
 // us per step of bands with R = 1, 2, 4 rows per warp (B200, FP32, 16 warps): run,
 // recorded run, reverse sweep
-constexpr double STEP_US[3][3] = {{0.79, 1.04, 1.82}, {0.95, 1.35, 4.0}, {1.4, 2.6, 0.0}};
+constexpr double STEP_US[3][3] = {{0.82, 1.06, 1.66}, {1.0, 1.5, 4.0}, {1.4, 2.6, 0.0}};
 
 // The CTAs by the steps they have been given, fewest first.
 struct Loads {
@@ -90,8 +90,9 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
     return G;
   };
   // The rows per warp with which the last CTA is done first: more rows are fewer and
-  // slower turns (96 x 256^2, 2000 steps: 38 / 23 / 22 ms with R = 1 / 2 / 4; 12
-  // recorded grids of 100^2 to 512^2: 3.8 / 2.8 / 3.9 ms)
+  // slower turns (96 x 256^2, 2000 steps: 40 / 23 / 20 ms with R = 1 / 2 / 4; 12
+  // recorded grids of 100^2 to 512^2: 3.9 / 3.2 / 3.9 ms, of 100^2 to 200^2 0.84 / 1.24 /
+  // 3.3; their sweeps 5.5 / 5.3 and 1.3 / 2.2)
   bool record = false;
   for (int b = 0; b < n; ++b) record = record || insts[b].curl != nullptr;
   int R = 0;
