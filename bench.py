@@ -895,7 +895,8 @@ def run_fdtd2d(args):
             "grid_1024": out["1024"],
             "roofline": {"bound": "hbm", "achieved": out["1024"]["gbs"], "peak": peak,
                          "unit": "GB/s", "frac": out["1024"]["gbs"] / peak,
-                         "note": "1024^2 grid (28 B/cell-step); 256^2 is L2-resident"},
+                         "note": "1024^2 grid, as if every step moved its 28 B/cell; the run "
+                                 "keeps its fields in registers, so this may exceed 1"},
             "e2e": out["e2e"], "cpu_baseline": cpu,
             "fp64_check": c0.get("fp64_check"),
             "gpu_launches": c0_launches,
