@@ -63,6 +63,11 @@ class DnCurlRecord(ctypes.Structure):
                 ("nslots", c_int32)]
 
 
+class DnResidentPlan(ctypes.Structure):
+    _fields_ = [("rows", c_int32), ("bands", c_int32), ("cluster", c_int32), ("pieces", c_int32),
+                ("shortest", c_int32), ("longest", c_int32)]
+
+
 class DnBatch2dInst(ctypes.Structure):
     _fields_ = [("H", c_int32), ("W", c_int32), ("pitch", c_int64), ("n_steps", c_int32),
                 ("src_comp", c_int32), ("src_box", DnBox), ("wave", c_void_p),
@@ -113,6 +118,7 @@ DN_MAX_SPANS = 32
 
 STRUCTS = {"dn_box": DnBox, "dn_grid": DnGrid, "dn_cpml": DnCpml, "dn_source": DnSource,
            "dn_monitor": DnMonitor, "dn_probe": DnProbe, "dn_curl_record": DnCurlRecord,
+           "dn_resident_plan": DnResidentPlan,
            "dn_batch2d_inst": DnBatch2dInst, "dn_batch2d": DnBatch2d,
            "dn_gemm_operand": DnGemmOperand, "dn_gemm": DnGemm,
            "dn_density": DnDensity, "dn_span": DnSpan}
@@ -137,6 +143,12 @@ SIGNATURES = {
                                    ctypes.POINTER(DnMonitor), c_int32, ctypes.POINTER(DnProbe),
                                    ctypes.POINTER(DnCurlRecord), c_int32, c_int32, c_void_p,
                                    c_void_p, ctypes.POINTER(c_int32), c_void_p, c_int64]),
+    "dn_fdtd2d_resident_plan": (c_int32, [ctypes.POINTER(DnGrid), ctypes.POINTER(DnSource),
+                                          ctypes.POINTER(DnMonitor), c_int32, c_int32, c_int32,
+                                          c_int32, ctypes.POINTER(DnResidentPlan)]),
+    "dn_fdtd3d_resident_plan": (c_int32, [ctypes.POINTER(DnGrid), ctypes.POINTER(DnSource),
+                                          ctypes.POINTER(DnMonitor), c_int32, c_int32, c_int32,
+                                          ctypes.POINTER(DnResidentPlan)]),
     "dn_fdtd3d_workspace_bytes": (c_int64, [ctypes.POINTER(DnGrid), ctypes.POINTER(DnSource),
                                             ctypes.POINTER(DnMonitor), c_int32, c_int32]),
     "dn_fdtd3d_run_ws": (c_int32, [ctypes.POINTER(DnGrid), _P6, _P6, c_void_p,

@@ -39,6 +39,7 @@ extern "C" int64_t dn_struct_size(const char* name) {
       {"dn_cpml", sizeof(dn_cpml)},       {"dn_source", sizeof(dn_source)},
       {"dn_monitor", sizeof(dn_monitor)}, {"dn_probe", sizeof(dn_probe)},
       {"dn_curl_record", sizeof(dn_curl_record)},
+      {"dn_resident_plan", sizeof(dn_resident_plan)},
       {"dn_batch2d_inst", sizeof(dn_batch2d_inst)},
       {"dn_batch2d", sizeof(dn_batch2d)},
       {"dn_gemm_operand", sizeof(dn_gemm_operand)},

@@ -31,6 +31,38 @@ inline unsigned used_mask(bool is3d, int pol) {
                       : ((1u << DN_HZ) | (1u << DN_EX) | (1u << DN_EY));
 }
 
+// SMs of the current device, 0 when it cannot be asked
+inline int sm_count() {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 0;
+  return nsm;
+}
+
+// A resident run of n steps as launches of at most `most` steps, all of nearly the
+// same length: floor(n / count) or one more, so never a single step while most >= 2.
+// (A launch reads and writes the same fields, and what keeps a band from storing rows
+// that a neighbour still has to load is the exchange between its first and its second
+// step.)
+struct Pieces {
+  int n, count;
+  Pieces(int n_, int most) : n(n_), count(most > 0 ? (int)(((long long)n_ + most - 1) / most) : 0) {}
+  int begin(int q) const { return (int)((long long)n * q / count); }
+};
+
+inline int describe_pieces(int nsteps, int most, dn_resident_plan* out) {
+  const Pieces cut(nsteps, most);
+  out->pieces = cut.count;
+  out->shortest = nsteps;
+  for (int q = 0; q < cut.count; ++q) {
+    const int k = cut.begin(q + 1) - cut.begin(q);
+    out->shortest = out->shortest < k ? out->shortest : k;
+    out->longest = out->longest > k ? out->longest : k;
+  }
+  return DN_OK;
+}
+
 // Launch on stream s; `chained`: as a dependent launch of the kernel launched
 // before it on s, which must pass pdl_release() and which this one waits for in
 // pdl_wait() before it touches anything a kernel of the chain writes.

@@ -41,7 +41,8 @@ Split choose_split(int H, int W, int elem, int nsm, int r_max) {
 }
 
 constexpr long long SAMPLE_BYTES = 64LL << 20;  // most workspace for samples
-constexpr int MIN_STEPS = 8;  // shorter runs (or pieces between DFTs) go launch by launch
+constexpr int MIN_STEPS = 8;  // shorter runs go launch by launch
+constexpr int MIN_PIECE = 4 * MIN_STEPS;  // so do runs whose samples allow fewer steps per launch
 
 // everything a run needs, or ok = false for the launch-by-launch path
 struct Plan2d {
@@ -49,16 +50,13 @@ struct Plan2d {
   Split S;
   long long mail_bytes;    // the two mailboxes of every band
   long long sample_bytes;  // one step's samples of all monitors
-  int piece;               // steps per launch (whole run, or what the samples allow)
+  int piece;               // most steps per launch (whole run, or what the samples allow)
 };
 
 Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mons, int n_mon,
-                   int nsteps, bool adjoint) {
+                   int nsteps, bool adjoint, int nsm = sm_count()) {
   Plan2d P{};
-  int dev = 0, nsm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return P;
+  if (nsm < 1) return P;
   const int elem = g->dtype == DN_F32 ? 4 : 8;
   const int first = g->pol == DN_TM ? DN_EZ : DN_HZ;
   if (nsteps < MIN_STEPS || (g->pitch_y * elem) % 16 != 0) return P;
@@ -77,7 +75,7 @@ Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mon
     P.sample_bytes += (to_dev(mons[m].box).cells() * elem + 15) / 16 * 16;
   if (P.sample_bytes * nsteps > SAMPLE_BYTES) {
     P.piece = (int)(SAMPLE_BYTES / P.sample_bytes);
-    if (P.piece < 4 * MIN_STEPS) return P;
+    if (P.piece < MIN_PIECE) return P;
   }
   P.ok = true;
   return P;
@@ -110,8 +108,9 @@ int run2d_resident(const dn_grid* g, void* const fa[6], void* const fb[6], const
   J.src = p.src.comp >= 0;
   J.wave = p.src.wave;
   constexpr int VEC = 16 / (int)sizeof(T);
-  for (int n = 0; n < nsteps; n += P.piece) {
-    const int k = std::min(P.piece, nsteps - n);
+  const Pieces cut(nsteps, P.piece);
+  for (int piece = 0; piece < cut.count; ++piece) {
+    const int n = cut.begin(piece), k = cut.begin(piece + 1) - n;
     J.t0 = t0 + n;
     J.nsteps = k;
     for (int c = 0; c < 3; ++c) {
@@ -267,8 +266,9 @@ int adjoint_ws(const dn_grid* g, void* const la[6], void* const lb[6], const voi
   J.grad = grad;
   J.curl_stride = curl->step_stride;
   constexpr int VEC = 16 / (int)sizeof(T);
-  for (int n = 0; n < nsteps; n += P.piece) {
-    const int k = std::min(P.piece, nsteps - n);
+  const Pieces cut(nsteps, P.piece);
+  for (int piece = 0; piece < cut.count; ++piece) {
+    const int n = cut.begin(piece), k = cut.begin(piece + 1) - n;
     const int t = t_end - 1 - n;  // the piece's first reverse step
     J.nsteps = k;
     J.curl = static_cast<const T*>(curl->curl[2]) + (long long)(t - curl->t0) * J.curl_stride;
@@ -348,6 +348,23 @@ extern "C" int64_t dn_fdtd2d_workspace_bytes(const dn_grid* g, const dn_source* 
   return std::max(
       dn::res::workspace_of(dn::res::make_plan2d(g, src, mons, n_mon, nsteps, false)),
       dn::res::workspace_of(dn::res::make_plan2d(g, nullptr, mons, n_mon, nsteps, true)));
+}
+
+extern "C" int32_t dn_fdtd2d_resident_plan(const dn_grid* g, const dn_source* src,
+                                           const dn_monitor* mons, int32_t n_mon, int32_t nsteps,
+                                           int32_t adjoint, int32_t n_sm, dn_resident_plan* out) {
+  if (!out || n_sm < 0 || nsteps < 0 ||
+      dn_fdtd2d_workspace_bytes(g, src, mons, n_mon, nsteps) < 0)
+    return DN_EINVAL;
+  *out = dn_resident_plan{};
+  const dn::res::Plan2d P =
+      dn::res::make_plan2d(g, adjoint ? nullptr : src, mons, n_mon, nsteps, adjoint != 0,
+                           n_sm > 0 ? n_sm : dn::sm_count());
+  if (!P.ok) return DN_OK;
+  out->rows = P.S.R;
+  out->bands = P.S.bands;
+  out->cluster = P.S.cluster;
+  return dn::describe_pieces(nsteps, P.piece, out);
 }
 
 extern "C" int32_t dn_fdtd2d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],

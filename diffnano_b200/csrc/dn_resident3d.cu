@@ -475,26 +475,23 @@ __global__ void __launch_bounds__(NT, 1) k_resident3d(const __grid_constant__ Jo
 
 // ---- host -----------------------------------------------------------------------------------
 constexpr long long SAMPLE_BYTES = 64LL << 20;  // most workspace for samples
-constexpr int MIN_STEPS = 8;  // shorter runs (or pieces between DFTs) go launch by launch
+constexpr int MIN_STEPS = 8;  // shorter runs go launch by launch
+constexpr int MIN_PIECE = 4 * MIN_STEPS;  // so do runs whose samples allow fewer steps per launch
 
 struct Plan {
   bool ok;
   int bz, by, nz, ny, smem;
   long long word_bytes;    // both sets of the rows on their way
   long long sample_bytes;  // one step's samples of all monitors
-  int piece;               // steps per launch
+  int piece;               // most steps per launch
 };
 
 // Blocks of rows, at most one per SM: among the splits whose largest block fits in
 // shared memory, the one with the fewest turns of the threads through its three
 // passes over rows, then with the fewest rows to update and to take per step.
 Plan make_plan(const dn_grid* g, const dn_source* src, const dn_monitor* mons, int n_mon,
-               int nsteps) {
+               int nsteps, int nsm = sm_count()) {
   Plan P{};
-  int dev = 0, nsm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return P;
   if (g->dtype != DN_F32 || nsteps < MIN_STEPS || g->W > 4 * NT || g->D > 0x7fff || g->H > 0x7fff)
     return P;
   if (src && src->component != DN_NONE && src->component > DN_EZ) return P;
@@ -527,7 +524,7 @@ Plan make_plan(const dn_grid* g, const dn_source* src, const dn_monitor* mons, i
     P.sample_bytes += (to_dev(mons[m].box).cells() * 4 + 15) / 16 * 16;
   if (P.sample_bytes * nsteps > SAMPLE_BYTES) {
     P.piece = (int)(SAMPLE_BYTES / P.sample_bytes);
-    if (P.piece < 4 * MIN_STEPS) return P;
+    if (P.piece < MIN_PIECE) return P;
   }
   P.ok = true;
   return P;
@@ -602,8 +599,9 @@ int run(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
   J.words = reinterpret_cast<uint4*>(ws);
   J.status = status;
   if (rec) J.curl_stride = rec->step_stride;
-  for (int n = 0; n < nsteps; n += P.piece) {
-    const int k = std::min(P.piece, nsteps - n);
+  const Pieces cut(nsteps, P.piece);
+  for (int piece = 0; piece < cut.count; ++piece) {
+    const int n = cut.begin(piece), k = cut.begin(piece + 1) - n;
     J.nsteps = k;
     if (J.src >= 0) J.wave = p.src.wave + t0 + n;
     for (int c = 0; c < 6; ++c) {
@@ -668,6 +666,21 @@ extern "C" int64_t dn_fdtd3d_workspace_bytes(const dn_grid* g, const dn_source* 
   for (int m = 0; m < n_mon; ++m)
     if (!dn::box_ok(mons[m].box, g->D, g->H, g->W)) return -1;
   return dn::res3::workspace_of(dn::res3::make_plan(g, src, mons, n_mon, nsteps));
+}
+
+extern "C" int32_t dn_fdtd3d_resident_plan(const dn_grid* g, const dn_source* src,
+                                           const dn_monitor* mons, int32_t n_mon, int32_t nsteps,
+                                           int32_t n_sm, dn_resident_plan* out) {
+  if (!out || n_sm < 0 || nsteps < 0 ||
+      dn_fdtd3d_workspace_bytes(g, src, mons, n_mon, nsteps) < 0)
+    return DN_EINVAL;
+  *out = dn_resident_plan{};
+  const dn::res3::Plan P =
+      dn::res3::make_plan(g, src, mons, n_mon, nsteps, n_sm > 0 ? n_sm : dn::sm_count());
+  if (!P.ok) return DN_OK;
+  out->rows = P.nz * P.ny;
+  out->bands = P.bz * P.by;
+  return dn::describe_pieces(nsteps, P.piece, out);
 }
 
 extern "C" int32_t dn_fdtd3d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],

@@ -185,6 +185,20 @@ int32_t dn_fdtd2d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],
                          int32_t t0, int32_t nsteps, int32_t* status, void* stream,
                          int32_t* final_in_b, void* ws, int64_t ws_bytes);
 
+/* How dn_fdtd2d_run_ws (adjoint = 0) or dn_fdtd2d_adjoint_ws (adjoint = 1) takes
+ * `nsteps` steps of this grid, given workspace enough, on a GPU of n_sm
+ * multiprocessors (0: the current device).  rows = 0: launch by launch. */
+typedef struct {
+  int32_t rows;      /* rows of the grid per warp (3-D: per CTA, planes x rows) */
+  int32_t bands;     /* CTAs that hold the grid */
+  int32_t cluster;   /* 1: the CTAs are one thread-block cluster */
+  int32_t pieces;    /* launches, as the monitors' samples allow ... */
+  int32_t shortest, longest; /* ... and their steps */
+} dn_resident_plan;
+int32_t dn_fdtd2d_resident_plan(const dn_grid* g, const dn_source* src, const dn_monitor* mons,
+                                int32_t n_mon, int32_t nsteps, int32_t adjoint, int32_t n_sm,
+                                dn_resident_plan* out);
+
 /* 3-D analogue (all six components), same ping-pong and status contract.
  * Field bases and ce must be 16-byte aligned, pitches multiples of 16 bytes. */
 int32_t dn_fdtd3d_run(const dn_grid* g, void* const fa[6], void* const fb[6], const void* ce,
@@ -203,6 +217,9 @@ int32_t dn_fdtd3d_run_ws(const dn_grid* g, void* const fa[6], void* const fb[6],
                          int32_t n_mon, const dn_probe* probe, const dn_curl_record* rec,
                          int32_t t0, int32_t nsteps, int32_t* status, void* stream,
                          int32_t* final_in_b, void* ws, int64_t ws_bytes);
+int32_t dn_fdtd3d_resident_plan(const dn_grid* g, const dn_source* src, const dn_monitor* mons,
+                                int32_t n_mon, int32_t nsteps, int32_t n_sm,
+                                dn_resident_plan* out);
 
 /* ---- adjoint (reverse) time stepping ------------------------------------
  * Discrete adjoint of the steps above: runs reverse steps t = t_end-1 down
