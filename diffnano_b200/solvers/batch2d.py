@@ -176,9 +176,9 @@ class FDTDBatch2D:
         sqrt of the longest step count, or no stored states at all where the
         curl terms of all steps can be recorded)
     tile_rows : 8, 16 or 32; None lets ``autotune_tile_rows`` choose
-    cluster : gradient-free solves that do not run resident, with each grid in
-        one 16-CTA thread-block cluster: None = when every grid fits, False =
-        never, True = always (error if a grid does not fit)
+    cluster : gradient-free solves with each grid in one 16-CTA thread-block
+        cluster: None = when every grid fits and the batch cannot run resident,
+        False = never, True = always (error if a grid does not fit)
     """
 
     def __init__(self, instances, polarization: str = "TM", dtype=torch.float32,
@@ -236,7 +236,8 @@ class FDTDBatch2D:
         self._graph = None
         if self._auto_rows:
             self.tile_rows = 16
-        self._plan_resident()
+        if grad or not self.cluster:
+            self._plan_resident()
         if self._record and (False not in self._plans or True not in self._plans):
             self._record = False  # some grid does not fit on the chip
             self._make_insts(grad, views, record=False)
@@ -285,7 +286,9 @@ class FDTDBatch2D:
 
     def uses_resident(self, fwd: bool, grad: bool) -> bool:
         """Whether a forward (with or without gradient) or backward run keeps the
-        grids on the chip."""
+        grids on the chip (``cluster=True`` asks for the cluster kernel instead)."""
+        if fwd and not grad and self.cluster:
+            return False
         return (not fwd) in self._plans and (self._record or not grad)
 
     def _stacked_views(self):
@@ -344,7 +347,7 @@ class FDTDBatch2D:
 
     def uses_cluster(self, grad: bool) -> bool:
         """Whether the batch fits the cluster kernel and may use it for a forward with /
-        without gradient (a resident plan comes first)."""
+        without gradient (a resident plan comes first unless ``cluster=True``)."""
         return (not grad) and self.cluster is not False and self._cluster[0] > 0
 
     def _launch(self, fwd: bool, grad: bool = True):
