@@ -153,6 +153,31 @@ class _Inst:
         return s
 
 
+def fits_cluster(spec: BatchInstance, polarization: str, dtype) -> bool:
+    """Whether a grid fits the cluster kernel (asked on the host: any non-null addresses
+    do)."""
+    pol = _lib.DN_TM if polarization.upper() == "TM" else _lib.DN_TE
+    H, W = spec.grid_shape
+    some = 16
+    inst = _lib.DnBatch2dInst(H=H, W=W, pitch=padded_width(W), n_steps=spec.n_steps,
+                              src_comp=_lib.DN_NONE, ce=some, dt=spec.dt, dl=spec.dl,
+                              mon_comp=_lib.DN_NONE, phase=some, acc=some)
+    for a in range(2):
+        inst.b[a] = inst.c[a] = some
+        for c in range(3):
+            inst.f[a][c] = some
+    if spec.monitor is not None:
+        box = _setup.monitor_box(spec.monitor, (1, H, W), False)
+        inst.mon_comp = _lib.DN_EZ if pol == _lib.DN_TM else _lib.DN_HZ
+        inst.mon_box = _lib.box([a for a, _ in box], [b for _, b in box])
+        inst.n_freq = len(spec.monitor.get("wavelengths_nm", [spec.wavelength_nm]))
+    cfg = _lib.DnBatch2d(pol=pol, dtype=_lib.DN_F32 if dtype == torch.float32 else _lib.DN_F64,
+                         n_inst=1, K=1, tile_rows=16)
+    smem = ctypes.c_int64(0)
+    return int(_lib.lib().dn_batch2d_cluster_size(ctypes.byref(cfg), ctypes.byref(inst),
+                                                  ctypes.byref(smem))) > 0
+
+
 def _signature(specs, pol, dtype) -> str:
     key = json.dumps([pol, str(dtype)] + [[*s.grid_shape, s.n_steps] for s in specs])
     return hashlib.sha1(key.encode()).hexdigest()[:16]

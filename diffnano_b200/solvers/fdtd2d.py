@@ -3,7 +3,9 @@
 Same constructor, attributes, ``forward`` and ``time_series`` as the
 reference (``diffnano/solvers/fdtd2d.py:91-524``); every time step runs in the
 CUDA kernels behind ``dn_fdtd2d_run_ws`` (``include/dn_fdtd.h``): grids that fit on
-the chip take all steps in one launch, larger ones one launch per step.  Additions, all
+the chip take all steps in one launch, larger ones one launch per step; solves without
+gradient that it would step launch by launch (FP32 TE, a few steps) run in one
+thread-block cluster where that is faster.  Additions, all
 optional keyword arguments: ``backward`` ("auto"/"autograd"/"time_reversal"/
 "checkpoint"), ``dtype`` (torch.float32 default, torch.float64 for
 validation), and DFT ``monitors``.
@@ -14,6 +16,7 @@ from __future__ import annotations
 import json
 import math
 from collections.abc import Sequence
+from types import SimpleNamespace
 
 import torch
 
@@ -25,7 +28,12 @@ from diffnano_b200.solvers._common import (
     monitor_metadata,
     parse_monitors,
 )
-from diffnano_b200.solvers._engine import Engine, compute_device, to_result_device
+from diffnano_b200.solvers._engine import (
+    Engine,
+    compute_device,
+    runs_resident_2d,
+    to_result_device,
+)
 from diffnano_b200.solvers._result import SimResult
 
 __all__ = ["FDTDSolver2D"]
@@ -117,19 +125,27 @@ class FDTDSolver2D:
         eps = self._prep_eps(geometry)
         mons = monitors if monitors is not None else self.monitors
         probe = src.get("probe", None)
-        from diffnano_b200.solvers._adjoint import run_forward
-
         needs_grad = torch.is_grad_enabled() and eps.requires_grad
-        eng = self._engine_for(src, mons, probe, reuse=not needs_grad)
-        field, dfts = run_forward(self, eng, eps, self._fields()[0])
+        fast = None
+        if probe is None and not needs_grad and not self._resident():
+            fast = self._cluster_solve(eps, src, mons)
+        if fast is not None:
+            specs, field, dfts = fast
+        else:
+            from diffnano_b200.solvers._adjoint import run_forward
+
+            eng = self._engine_for(src, mons, probe, reuse=not needs_grad)
+            specs = eng.monitors
+            field, dfts = run_forward(self, eng, eps, self._fields()[0])
         out_dev = self._device
         snapshots = []
         if probe is not None:
             snapshots = list(eng.probe_out.to(out_dev, copy=True).unbind(0))
         meta = {"polarization": self.polarization, "n_steps": self.n_steps, "dt": self.dt,
                 "courant": self.courant, "snapshots": snapshots}
-        if eng.monitors:
-            meta["monitors"] = monitor_metadata(eng, [to_result_device(d, out_dev) for d in dfts])
+        if specs:
+            meta["monitors"] = monitor_metadata(SimpleNamespace(monitors=specs),
+                                                [to_result_device(d, out_dev) for d in dfts])
         return SimResult(field=to_result_device(field.unsqueeze(0), out_dev), wavelengths=wl,
                          metadata=meta)
 
@@ -142,20 +158,80 @@ class FDTDSolver2D:
         (tensors in the source or monitor dicts) are not cached."""
         if not reuse:
             return self._make_engine(self.n_steps, src, mons, probe)
+        return self._kept("_engine_cache", src, mons, probe,
+                          lambda: self._make_engine(self.n_steps, src, mons, probe))
+
+    def _kept(self, name: str, src: dict, mons, probe, make):
+        """``make()``, or what it made for the same set-up before (the last four)."""
         try:
             key = json.dumps([src, mons, probe, self.n_steps, str(self.dtype),
                               list(self.grid_shape), self.dl, self.wavelength_nm,
                               self.pml_layers, self.courant, self.polarization,
                               str(self._device)], sort_keys=True)
         except TypeError:
-            return self._make_engine(self.n_steps, src, mons, probe)
-        cache = self.__dict__.setdefault("_engine_cache", {})
-        eng = cache.get(key)
-        if eng is None:
+            return make()
+        cache = self.__dict__.setdefault(name, {})
+        if key not in cache:
             if len(cache) >= 4:
                 cache.clear()
-            eng = cache[key] = self._make_engine(self.n_steps, src, mons, probe)
-        return eng
+            cache[key] = make()
+        return cache[key]
+
+    def _resident(self) -> bool:
+        """Whether a solve of this set-up runs resident."""
+        key = (tuple(self.grid_shape), self.dtype, self.polarization, self.n_steps,
+               str(self._device))
+        known = self.__dict__.setdefault("_resident_known", {})
+        if key not in known:
+            known.clear()
+            known[key] = runs_resident_2d(self.grid_shape, self.dtype,
+                                          _lib.DN_TM if self.polarization == "TM" else _lib.DN_TE,
+                                          self.n_steps, compute_device(self._device))
+        return known[key]
+
+    def _cluster_solve(self, eps, src, mons):
+        """Gradient-free solve with the whole grid in one thread-block cluster
+        (``dn_batch2d_forward_cluster``) when the grid fits and there is at most
+        one monitor, on the injected field: (monitor specs, field, DFTs), else
+        None."""
+        H, W = self.grid_shape
+        specs = parse_monitors(mons, (1, H, W), False, self.wavelength_nm, self._fields()[0],
+                               self._fields())
+        batch = self._kept("_cluster_cache", src, mons, None,
+                           lambda: self._make_cluster(src, specs))
+        if batch is None:
+            return None
+        with torch.no_grad():
+            fields, dfts = batch.run_forward([eps], grad=False)
+        batch.check_status()
+        return specs, fields[0], [d for d in dfts if d is not None]
+
+    def _make_cluster(self, src: dict, specs):
+        """The batch of one that ``_cluster_solve`` runs, None when it cannot or would be
+        slower.  A step of the cluster kernel costs what its busiest warp walks, a row in
+        pieces of 32 columns: us per step in the cluster, B200, where a launch per step
+        takes 6.2: 64^2 0.8, 100^2 2.5, 256^2 2.9, 270 x 333 5.2 (22 pieces), 256 x 512
+        5.8 (16); 460 x 400 7.7 (26), 64 x 1024 7.3 (32), 64 x 2100 20.6 (66)."""
+        from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D, fits_cluster
+
+        H, W = self.grid_shape
+        rows = -(-H // 16)  # per CTA, 16 warps each
+        if -(-rows // 16) * -(-W // 32) > 24:
+            return None
+        mon = None
+        if len(specs) > 1 or (specs and specs[0].component !=
+                              _lib.COMPONENTS[self._fields()[0]]):
+            return None
+        if specs:
+            m = specs[0]
+            mon = {"box": [list(m.box[1]), list(m.box[2])], "wavelengths_nm": list(m.wavelengths)}
+        spec = BatchInstance(grid_shape=tuple(self.grid_shape), n_steps=self.n_steps, dl=self.dl,
+                             wavelength_nm=self.wavelength_nm, pml_layers=self.pml_layers,
+                             courant=self.courant, source=dict(src), monitor=mon)
+        if not fits_cluster(spec, self.polarization, self.dtype):
+            return None
+        return FDTDBatch2D([spec], self.polarization, self.dtype, compute_device(self._device),
+                           tile_rows=16, cluster=True)
 
     def time_series(self, eps_r: torch.Tensor, probe: tuple[int, int], source: dict | None = None,
                     n_steps: int | None = None) -> torch.Tensor:
