@@ -8,7 +8,7 @@ both modes are one ``torch.autograd.Function`` whose backward is the discrete
 adjoint of the kernels' own step:
 
 * forward: all T steps run in the CUDA kernels.  When a gradient is needed and
-  the curl terms of all T steps fit an eighth of the GPU's memory, they are
+  there is room for the curl terms of all T steps (``_records``), they are
   recorded as the steps run; else (and whenever the caller asks for
   checkpoints) the state is copied every K steps (K = sqrt(T), or T /
   checkpoint_segments with ``use_checkpoint``);
@@ -29,10 +29,10 @@ from __future__ import annotations
 import torch
 
 from diffnano_b200 import _lib
+from diffnano_b200.solvers import _records
 from diffnano_b200.solvers._common import checkpoint_interval
 
 F64 = torch.float64
-RECORD_SHARE = 1 / 8  # of the GPU's memory, for the curl terms of all steps
 
 
 def _outputs(eng, out_names):
@@ -51,22 +51,21 @@ class _Runner:
         self.K = max(1, int(interval))
         self.checkpoints = {}
         self.full_record = full_record  # try to record every step's curl terms
-        self.curl = None
+        self.record = None
 
     def forward(self, eps_dev: torch.Tensor, save: bool):
         eng = self.eng
         eng.reset()
         eng.set_eps(eps_dev)
         T, K = eng.n_steps, self.K
-        if save and self.full_record and eng.curl_bytes(T) <= RECORD_SHARE * \
-                torch.cuda.get_device_properties(eng.device).total_memory:
-            try:
-                self.curl = eng.curl_buffer(T)
-            except torch.OutOfMemoryError:
-                self.curl = None  # checkpoints need less
+        if save and self.full_record:
+            # beside it: two adjoint states, the FP64 gradient, the outputs
+            beside = 3 * eng.A.nbytes + 8 * eng.ce.numel()
+            self.record = _records.claim(eng.device, eng.curl_bytes(T), beside,
+                                         lambda: eng.curl_buffer(T))
         t = 0
-        if self.curl is not None:
-            eng.run(0, T, record=eng.curl_record(self.curl, 0, T))
+        if self.record is not None:
+            eng.run(0, T, record=eng.curl_record(self.record.made, 0, T))
             t = T
         while t < T:
             n = min(K, T - t)
@@ -113,8 +112,8 @@ class _Runner:
         n_mon = len(eng.monitors) if g_mon is not None else 0
         grad_ce = torch.zeros((D, H, eng.Wp), dtype=F64, device=eng.device)
         T, K = eng.n_steps, self.K
-        if self.curl is not None:
-            rec = eng.curl_record(self.curl, 0, T)
+        if self.record is not None:
+            rec = eng.curl_record(self.record.made, 0, T)
             eng.adjoint(la, lb, rec, grad_ce, mon_arr, n_mon, T, T)
             eng.check_status(extra=(grad_ce[..., :W],))
             return grad_ce[..., :W]

@@ -9,8 +9,8 @@ advances all of them in one persistent cooperative kernel
 (``dn_batch2d_backward``: checkpoint-segment replay + reverse steps), with the
 same step arithmetic as the single-grid kernels.  TM batches whose grids fit on
 the chip run grid by grid with the fields in registers instead
-(``dn_batch2d_run_resident``): always without a gradient, and with one where the
-curl terms of all steps fit an eighth of the GPU's memory (and no
+(``dn_batch2d_run_resident``): always without a gradient, and with one where there
+is room for the curl terms of all steps (``_records``; and no
 ``checkpoint_interval`` was asked for).  Each instance is described
 by the reference's own constructor arguments and source dict, plus one DFT
 line/point/box monitor on its injected field.
@@ -40,11 +40,10 @@ from dataclasses import dataclass, field
 import torch
 
 from diffnano_b200 import _lib
-from diffnano_b200.solvers import _setup
+from diffnano_b200.solvers import _records, _setup
 from diffnano_b200.solvers._engine import compute_device, padded_width
 
 F64 = torch.float64
-RECORD_SHARE = 1 / 8  # of the GPU's memory, for the curl terms of all steps
 
 
 @dataclass
@@ -224,7 +223,7 @@ class FDTDBatch2D:
         self.tile_rows = tile_rows
         self._auto_rows = tile_rows is None
         self._asked_checkpoints = checkpoint_interval is not None
-        self._record = False
+        self._record = None  # room for the curl terms of all steps, or None
         self._plans: dict = {}  # adjoint? -> (host plan, device plan, workspace bytes)
         self._ws = None
         self._insts = None
@@ -247,15 +246,17 @@ class FDTDBatch2D:
     def _build(self, grad: bool):
         if self._insts is not None and self._grad_alloc == grad:
             return
-        self._insts, self._record, self._plans = None, False, {}
+        self._insts, self._record, self._plans = None, None, {}
         views = self._stacked_views()
-        if grad and self._can_record():
-            try:
-                self._make_insts(grad, views, record=True)
-                self._record = True
-            except torch.OutOfMemoryError:
-                self._insts = None  # checkpoints need less
-        if self._insts is None:
+        # a TM batch, no checkpoints asked for
+        if grad and self.pol == _lib.DN_TM and not self._asked_checkpoints:
+            size = 4 if self.dtype == torch.float32 else 8
+            cells = [s.grid_shape[0] * padded_width(s.grid_shape[1]) for s in self.specs]
+            # beside it: two states, two adjoint ones, dt/eps and the FP64 gradient
+            self._record = _records.claim(
+                self.device, size * sum(s.n_steps * n for s, n in zip(self.specs, cells)),
+                (13 * size + 8) * sum(cells), lambda: self._make_insts(grad, views, record=True))
+        if self._record is None:
             self._make_insts(grad, views, record=False)
         self._grad_alloc = grad
         self._graph = None
@@ -263,8 +264,8 @@ class FDTDBatch2D:
             self.tile_rows = 16
         if grad or not self.cluster:
             self._plan_resident()
-        if self._record and (False not in self._plans or True not in self._plans):
-            self._record = False  # some grid does not fit on the chip
+        if self._record is not None and (False not in self._plans or True not in self._plans):
+            self._record = self._insts = None  # some grid does not fit on the chip
             self._make_insts(grad, views, record=False)
         if self._auto_rows and not self.uses_resident(True, grad):
             self.tile_rows = autotune_tile_rows(self)
@@ -276,16 +277,6 @@ class FDTDBatch2D:
                              None if views is None else views[n], record)
                        for n, s in enumerate(self.specs)]
 
-    def _can_record(self) -> bool:
-        """Whether the curl terms of all steps may be recorded: a TM batch, no
-        checkpoints asked for, within their share of the memory."""
-        if self.pol != _lib.DN_TM or self._asked_checkpoints:
-            return False
-        size = 4 if self.dtype == torch.float32 else 8
-        need = sum(s.n_steps * s.grid_shape[0] * padded_width(s.grid_shape[1]) for s in self.specs)
-        total = torch.cuda.get_device_properties(self.device).total_memory
-        return need * size <= RECORD_SHARE * total
-
     def _plan_resident(self) -> None:
         """Plans of the resident forward run and (recorded) reverse sweep, where
         the batch can run that way."""
@@ -293,7 +284,7 @@ class FDTDBatch2D:
         arr = (_lib.DnBatch2dInst * len(self._insts))(*[i.struct(self.pol) for i in self._insts])
         cfg = self._cfg(self.tile_rows, len(self._insts), 0)
         with torch.cuda.device(self.device):
-            for adjoint in ((False, True) if self._record else (False,)):
+            for adjoint in ((False, True) if self._record is not None else (False,)):
                 n = int(L.dn_batch2d_resident_bytes(ctypes.byref(cfg), arr, int(adjoint)))
                 if n <= 0:
                     continue
@@ -314,7 +305,7 @@ class FDTDBatch2D:
         grids on the chip (``cluster=True`` asks for the cluster kernel instead)."""
         if fwd and not grad and self.cluster:
             return False
-        return (not fwd) in self._plans and (self._record or not grad)
+        return (not fwd) in self._plans and (self._record is not None or not grad)
 
     def _stacked_views(self):
         """Uniform batches (every instance with the same grid, step count, time
