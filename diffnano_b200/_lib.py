@@ -83,6 +83,11 @@ class DnBatch2d(ctypes.Structure):
                 ("tile_rows", c_int32), ("max_ctas", c_int32)]
 
 
+class DnBatch2dPlan(ctypes.Structure):
+    _fields_ = [("rows", c_int32), ("launches", c_int32), ("most_grids", c_int32),
+                ("wait_polls", c_int64)]
+
+
 class DnGemmOperand(ctypes.Structure):
     _fields_ = [("ptr", c_void_p), ("mn_major", c_int32), ("fold", c_int32), ("rows", c_int64),
                 ("k", c_int64), ("ld", c_int64), ("fold_stride", c_int64),
@@ -120,6 +125,7 @@ STRUCTS = {"dn_box": DnBox, "dn_grid": DnGrid, "dn_cpml": DnCpml, "dn_source": D
            "dn_monitor": DnMonitor, "dn_probe": DnProbe, "dn_curl_record": DnCurlRecord,
            "dn_resident_plan": DnResidentPlan,
            "dn_batch2d_inst": DnBatch2dInst, "dn_batch2d": DnBatch2d,
+           "dn_batch2d_plan": DnBatch2dPlan,
            "dn_gemm_operand": DnGemmOperand, "dn_gemm": DnGemm,
            "dn_density": DnDensity, "dn_span": DnSpan}
 
@@ -184,6 +190,9 @@ SIGNATURES = {
     "dn_batch2d_resident_pack": (c_int32, [ctypes.POINTER(DnBatch2d),
                                            ctypes.POINTER(DnBatch2dInst), c_int32, c_void_p,
                                            c_int64, ctypes.POINTER(c_int64)]),
+    "dn_batch2d_resident_plan": (c_int32, [ctypes.POINTER(DnBatch2d),
+                                           ctypes.POINTER(DnBatch2dInst), c_int32, c_int32,
+                                           ctypes.POINTER(DnBatch2dPlan)]),
     "dn_batch2d_run_resident": (c_int32, [ctypes.POINTER(DnBatch2d), c_void_p, c_void_p, c_void_p,
                                           c_void_p, c_int64, c_int32, c_void_p, c_void_p]),
     "dn_batch2d_cluster_size": (c_int32, [ctypes.POINTER(DnBatch2d), ctypes.POINTER(DnBatch2dInst),

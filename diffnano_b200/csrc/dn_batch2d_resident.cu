@@ -26,6 +26,7 @@ struct Group {
   long long o_start, o_jobs;  // byte offsets
   long long mail_words, sample_bytes;
   long long max_cells;        // largest monitor
+  double steps;               // of the longest list
 };
 constexpr int MAX_GROUPS = 256;
 struct Head {
@@ -69,13 +70,10 @@ struct Loads {
 };
 
 // false: some grid does not fit, or the batch is not a TM one
-bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint, Plan* P) {
+bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint, Plan* P,
+               int nsm = sm_count()) {
   const long long off = batch2d_inst_offset(cfg, insts);
-  if (off < 0 || cfg->pol != DN_TM) return false;
-  int dev = 0, nsm = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return false;
+  if (off < 0 || cfg->pol != DN_TM || nsm < 1) return false;
   const int n = cfg->n_inst, elem = cfg->dtype == DN_F32 ? 4 : 8, cols = 32 * 16 / elem;
   std::vector<int> order(n);
   std::iota(order.begin(), order.end(), 0);
@@ -150,6 +148,7 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
     g.count = k - g.first;
     g.mail_words = mail;
     g.sample_bytes = sample;
+    g.steps = loads.v.back().first;
     ws = std::max(ws, mail * 8 + sample);
     std::vector<int> start(nsm + 1, 0);
     std::vector<ListJob> jobs;
@@ -227,7 +226,8 @@ int run_groups(const Head& h, bool record, unsigned char* table, unsigned char* 
            reinterpret_cast<const ListJob*>(blob + g.o_jobs),
            reinterpret_cast<const int*>(blob + g.o_start),
            reinterpret_cast<uint64_t*>(ws),
-           ws + g.mail_words * 8};
+           ws + g.mail_words * 8,
+           polls_of(g.steps)};
     DN_CUDA_CHECK(cudaMemsetAsync(ws, 0, (size_t)g.mail_words * 8, s));
     const unsigned cells = (unsigned)((g.max_cells + 31) / 32);
     if (h.adjoint && cells) {
@@ -254,6 +254,24 @@ extern "C" int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_bat
   if (!cfg || !insts) return -1;
   dn::res::Plan P;
   return dn::res::make_plan(cfg, insts, adjoint != 0, &P) ? P.h.bytes : 0;
+}
+
+extern "C" int32_t dn_batch2d_resident_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                            int32_t adjoint, int32_t n_sm, dn_batch2d_plan* out) {
+  if (!cfg || !insts || !out || n_sm < 0 || dn::batch2d_inst_offset(cfg, insts) < 0)
+    return DN_EINVAL;
+  *out = dn_batch2d_plan{};
+  dn::res::Plan P;
+  if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P, n_sm > 0 ? n_sm : dn::sm_count()))
+    return DN_OK;
+  out->rows = P.h.R;
+  out->launches = P.h.n_groups;
+  for (int g = 0; g < P.h.n_groups; ++g) {
+    const dn::res::Group& G = P.h.group[g];
+    out->most_grids = std::max(out->most_grids, G.count);
+    out->wait_polls = std::max<int64_t>(out->wait_polls, dn::res::polls_of(G.steps));
+  }
+  return DN_OK;
 }
 
 extern "C" int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,

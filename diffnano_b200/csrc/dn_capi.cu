@@ -42,6 +42,7 @@ extern "C" int64_t dn_struct_size(const char* name) {
       {"dn_resident_plan", sizeof(dn_resident_plan)},
       {"dn_batch2d_inst", sizeof(dn_batch2d_inst)},
       {"dn_batch2d", sizeof(dn_batch2d)},
+      {"dn_batch2d_plan", sizeof(dn_batch2d_plan)},
       {"dn_gemm_operand", sizeof(dn_gemm_operand)},
       {"dn_gemm", sizeof(dn_gemm)},
       {"dn_density", sizeof(dn_density)},

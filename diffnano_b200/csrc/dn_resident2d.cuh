@@ -44,6 +44,18 @@ namespace res {
 
 enum { MAIL_CLUSTER = 0, MAIL_GLOBAL = 1 };
 
+// Polls of one wait on a global mailbox, a round trip to L2 (0.3 us and more) each.
+// All bands of a lone grid start together; in a batch a band that starts early waits
+// for a neighbour whose CTA still runs earlier grids, for as long as the whole launch
+// may take: POLLS_PER_STEP for each step of the longest list (a step takes up to
+// 4 us) come on top.
+constexpr unsigned SPIN_LIMIT = 1u << 22;
+constexpr unsigned POLLS_PER_STEP = 64;
+inline unsigned polls_of(double steps) {
+  const double p = SPIN_LIMIT + POLLS_PER_STEP * steps;
+  return p < 4e9 ? (unsigned)p : 4000000000u;
+}
+
 constexpr int MAX_WARPS = 16;  // warps per CTA: 128 registers each
 constexpr int ROW_WORDS = 4 * 32;  // 64-bit mailbox words per strip and row
 
@@ -131,6 +143,7 @@ struct List {
   const int* start;  // per CTA, its first job (and one past the last CTA's last)
   uint64_t* mail;
   unsigned char* samples;
+  unsigned polls;  // bound of one wait
 };
 
 // forward (adjoint = false) or reverse sweep of TM grids, R rows per warp

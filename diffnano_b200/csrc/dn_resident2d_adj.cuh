@@ -21,8 +21,8 @@ namespace res {
 
 template <typename T, int R, int MAIL>
 __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, int band,
-                                           unsigned char* smem, uint64_t* mail, int* status,
-                                           const Samples<T>* adds, int n_add) {
+                                           unsigned char* smem, uint64_t* mail, unsigned polls,
+                                           int* status, const Samples<T>* adds, int n_add) {
   using B = Block<T, R, MAIL>;
   using L = typename B::L;
   constexpr int VEC = B::VEC;
@@ -32,7 +32,7 @@ __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, i
   using C = typename V::S;
   const int H = J.H, W = J.W;
   const long long py = J.py;
-  const B K(H, W, S, band, smem, mail, status);
+  const B K(H, W, S, band, smem, mail, polls, status);
   const int lane = K.lane, ia = K.ia, j0 = K.j0, jv = K.jv;
   const bool live = K.live, any = K.any, full = K.full;
   const bool first_row = K.first_row, first_col = K.first_col, last_col = K.last_col;
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   if constexpr (MAIL == MAIL_CLUSTER) arm_mailboxes<L>(r_smem);
   const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
   if (!skip && (int)blockIdx.x < S.bands)
-    sweep_band<T, R, MAIL>(J, S, blockIdx.x, r_smem, mail, status, adds.s, adds.n);
+    sweep_band<T, R, MAIL>(J, S, blockIdx.x, r_smem, mail, SPIN_LIMIT, status, adds.s, adds.n);
   if constexpr (MAIL == MAIL_CLUSTER) cg::this_cluster().sync();  // no row still under way
 }
 

@@ -15,7 +15,6 @@ namespace res {
 namespace cg = cooperative_groups;
 
 constexpr unsigned ALL = STRIP_FULL_MASK;
-constexpr unsigned SPIN_LIMIT = 1u << 22;   // polls of one wait on a global mailbox
 constexpr unsigned PROBE_LIMIT = 1u << 16;  // probes of one wait on an mbarrier ...
 constexpr uint32_t PROBE_NS = 20000;        // ... each suspended for at most this long
 
@@ -185,13 +184,14 @@ __device__ __forceinline__ void post_words(uint64_t* box, uint32_t tag, const Pa
                  : "memory");
   }
 }
-// bounded wait for a row, or for two at once (TWO: both boxes are read in one
-// round trip); false when it gave up or another CTA recorded an error
+// bounded wait (about `polls`) for a row, or for two at once (TWO: both boxes are read
+// in one round trip); false when it gave up or another CTA recorded an error
 template <typename T, bool TWO>
 __device__ __forceinline__ bool take_words(const uint64_t* a, const uint64_t* b, uint32_t tag,
-                                           Pack<T>& va, Pack<T>& vb, const int* status) {
+                                           Pack<T>& va, Pack<T>& vb, unsigned polls,
+                                           const int* status) {
   constexpr int N = TWO ? 8 : 4;
-  for (unsigned n = 0; n < SPIN_LIMIT; ++n) {
+  for (unsigned n = 0;; ++n) {
     uint64_t u[N];
     bool ok = true;
 #pragma unroll
@@ -211,10 +211,10 @@ __device__ __forceinline__ bool take_words(const uint64_t* a, const uint64_t* b,
       }
       return true;
     }
-    if ((n & 4095u) == 4095u && status && *reinterpret_cast<const volatile int*>(status) != 0)
+    if ((n & 4095u) == 4095u &&
+        (n >= polls || (status && *reinterpret_cast<const volatile int*>(status) != 0)))
       return false;
   }
-  return false;
 }
 
 // shared-memory mailbox of a cluster neighbour: the lane's 16 bytes and their
@@ -324,6 +324,7 @@ struct Block {
   static constexpr int BAR_PAR = MAX_WARPS;  // mbarriers between the two slots
 
   unsigned char* smem;
+  unsigned polls;  // bound of one wait on a global mailbox
   int* status;
   int lane, w, strip, group, ia0, ia, j0, jv;
   bool active;  // has a block (a CTA may have more warps than a grid's bands use)
@@ -349,8 +350,9 @@ struct Block {
   long long slot;
 
   __device__ __forceinline__ Block(int H, int W, const Split& S, int band, unsigned char* smem_,
-                                   uint64_t* mail, int* status_) {
+                                   uint64_t* mail, unsigned polls_, int* status_) {
     smem = smem_;
+    polls = polls_;
     status = status_;
     lane = threadIdx.x & 31;
     w = threadIdx.x >> 5;
@@ -492,11 +494,11 @@ struct Block {
       if (!band_dn) f_dn = ld16<T>(dn_row + nxt * ROW_PAR);
       if (band_up && band_dn) {
         bad = !take_words<T, true>(in_up + nxt * slot, in_dn + nxt * slot, n + 1, f_up, f_dn,
-                                   status);
+                                   polls, status);
       } else if (band_up || band_dn) {
         V v, unused;
         bad = !take_words<T, false>((band_up ? in_up : in_dn) + nxt * slot, nullptr, n + 1, v,
-                                    unused, status);
+                                    unused, polls, status);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           f_up.p[h] = band_up ? v.p[h] : f_up.p[h];

@@ -12,8 +12,8 @@ namespace res {
 // ---------------------------------------------------------------------------
 template <typename T, int POL, int R, int MAIL, bool REC, bool SMP>
 __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int band,
-                                         unsigned char* smem, uint64_t* mail, int* status,
-                                         const Samples<T>* smps, int n_smp) {
+                                         unsigned char* smem, uint64_t* mail, unsigned polls,
+                                         int* status, const Samples<T>* smps, int n_smp) {
   using B = Block<T, R, MAIL>;
   using L = typename B::L;
   constexpr int VEC = B::VEC;
@@ -23,7 +23,7 @@ __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int ba
   const int H = J.H, W = J.W;
   const long long py = J.py;
   const double idl = 1.0 / J.dl;
-  const B K(H, W, S, band, smem, mail, status);
+  const B K(H, W, S, band, smem, mail, polls, status);
   const int lane = K.lane, ia = K.ia, j0 = K.j0, jv = K.jv;
   const bool live = K.live, any = K.any, full = K.full;
   const bool first_row = K.first_row, last_row = K.last_row;
@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   // a previous launch that recorded an error turns this one into a no-op
   const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
   if (!skip && (int)blockIdx.x < S.bands)
-    run_band<T, POL, R, MAIL, REC, SMP>(J, S, blockIdx.x, r_smem, mail, status, smps.s,
-                                   smps.n);
+    run_band<T, POL, R, MAIL, REC, SMP>(J, S, blockIdx.x, r_smem, mail, SPIN_LIMIT, status,
+                                             smps.s, smps.n);
   if constexpr (MAIL == MAIL_CLUSTER) cg::this_cluster().sync();  // no row still under way
 }
 

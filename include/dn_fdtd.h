@@ -359,6 +359,16 @@ int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* 
 int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                  int32_t adjoint, void* host_plan, int64_t bytes,
                                  int64_t* ws_bytes);
+/* How such a batch would be taken on a GPU of n_sm multiprocessors (0: the current
+ * device); rows = 0: not at all. */
+typedef struct {
+  int32_t rows;        /* rows per warp */
+  int32_t launches;
+  int32_t most_grids;  /* of a launch */
+  int64_t wait_polls;  /* bound of the longest wait for a neighbouring band, in round trips to L2 */
+} dn_batch2d_plan;
+int32_t dn_batch2d_resident_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
+                                 int32_t adjoint, int32_t n_sm, dn_batch2d_plan* out);
 int32_t dn_batch2d_run_resident(const dn_batch2d* cfg, void* dev_table, const void* host_plan,
                                 void* dev_plan, void* ws, int64_t ws_bytes, int32_t record,
                                 int32_t* status, void* stream);

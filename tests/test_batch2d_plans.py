@@ -1,0 +1,84 @@
+"""How TM batches are dealt to the chip (on the host, for a GPU of 148 multiprocessors),
+and the batches that a plan must not break."""
+
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+import torch
+from conftest import rel_l2
+
+from diffnano_b200 import _lib
+from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D
+
+SMS = 148
+SPIN_LIMIT, POLLS_PER_STEP = 1 << 22, 64
+
+
+def insts(grids, monitor=False):
+    """(H, W, steps) as the C ABI takes them; a plan looks at no address."""
+    arr = (_lib.DnBatch2dInst * len(grids))()
+    for n, (H, W, T) in enumerate(grids):
+        s = arr[n]
+        s.H, s.W, s.pitch, s.n_steps, s.dt, s.dl = H, W, (W + 31) // 32 * 32, T, 7.0, 20.0
+        s.src_comp = s.mon_comp = _lib.DN_NONE
+        s.ce = s.phase = s.acc = 16
+        for a in range(2):
+            s.b[a] = s.c[a] = 16
+            for c in range(3):
+                s.f[a][c] = 16
+        if monitor:
+            s.mon_comp, s.n_freq, s.mon_box = _lib.DN_EZ, 1, _lib.box((0, 0, 0), (1, 1, W))
+    cfg = _lib.DnBatch2d(pol=_lib.DN_TM, dtype=_lib.DN_F32, n_inst=len(grids), K=8, tile_rows=16)
+    return cfg, arr
+
+
+def plan(grids, monitor=False, adjoint=False):
+    cfg, arr = insts(grids, monitor)
+    out = _lib.DnBatch2dPlan()
+    _lib.check("plan", _lib.lib().dn_batch2d_resident_plan(ctypes.byref(cfg), arr, int(adjoint), SMS,
+                                                           ctypes.byref(out)))
+    return out
+
+
+# a band may wait for a CTA that still runs earlier grids: at most the whole launch
+@pytest.mark.parametrize("adjoint", [False, True])
+def test_waits_last_as_long_as_the_launch(adjoint):
+    p = plan([(100, 100, 900)] * 4, adjoint=adjoint)
+    assert p.rows > 0 and p.wait_polls == SPIN_LIMIT + POLLS_PER_STEP * 900
+    one = plan([(2368, 64, 8), (8, 8, 8_000_000)], adjoint=adjoint)
+    assert one.wait_polls >= SPIN_LIMIT + POLLS_PER_STEP * 8_000_000
+    many = plan([(256, 256, 2000)] * 2048, adjoint=adjoint)  # hundreds of grids per CTA
+    assert many.wait_polls >= SPIN_LIMIT + POLLS_PER_STEP * 2000 * (2048 * 8 // SMS)
+    endless = plan([(100, 100, 2_000_000_000)] * 300, adjoint=adjoint)
+    assert endless.wait_polls == 4_000_000_000  # bounded all the same
+
+
+def test_plans_reject_invalid_batches():
+    cfg, arr = insts([(100, 100, 900)])
+    out = _lib.DnBatch2dPlan()
+    call = _lib.lib().dn_batch2d_resident_plan
+    assert call(None, arr, 0, SMS, ctypes.byref(out)) == _lib.DN_EINVAL
+    arr[0].H = 0
+    assert call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out)) == _lib.DN_EINVAL
+    cfg.pol, arr[0].H = _lib.DN_TE, 100
+    assert call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out)) == _lib.DN_OK and out.rows == 0
+
+
+@pytest.mark.gpu
+def test_a_band_waits_out_a_long_run_on_its_neighbours_cta(cuda):
+    """One tiny grid of millions of steps on a CTA that a grid of a band per SM needs
+    too: its other bands wait for seconds."""
+    src = {"type": "gaussian_pulse", "row": 3, "spread": 100.0, "t0": 20.0}
+    long = BatchInstance(grid_shape=(8, 8), n_steps=8_000_000, pml_layers=2, source=src)
+    wide = BatchInstance(grid_shape=(16 * SMS, 64), n_steps=8, pml_layers=4,
+                         source={**src, "row": 16 * SMS // 2})
+    g = torch.Generator().manual_seed(2)
+    eps = [(1.5 + 2.0 * torch.rand(*s.grid_shape, dtype=torch.float64, generator=g)).to(cuda)
+           for s in (long, wide)]
+    b = FDTDBatch2D([long, wide], "TM", torch.float32, cuda, tile_rows=16)
+    fields, _ = b.forward(eps)
+    assert b.uses_resident(True, False)
+    alone, _ = FDTDBatch2D([wide], "TM", torch.float32, cuda, tile_rows=16).forward(eps[1:])
+    assert rel_l2(fields[1], alone[0]) < 1e-6 and float(alone[0].abs().max()) > 0
