@@ -16,8 +16,10 @@ long long batch2d_inst_offset(const dn_batch2d* cfg, const dn_batch2d_inst* inst
 namespace res {
 namespace {
 
-// samples of one launch (more grids than fit go in further launches)
+// samples of one launch, and grids (their monitors' kernels take one per blockIdx.y);
+// more go in further launches
 constexpr long long GROUP_SAMPLE_BYTES = 1LL << 30;
+constexpr int GROUP_GRIDS = 65535;
 
 // The blob: Head | ListGrid[n_inst] | per group: start[n_cta + 1], jobs | (host
 // and device copies are the same bytes).  Grids are in the table's order.
@@ -136,7 +138,8 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
         bytes = G.stride * elem * I.n_steps;
       }
       if (bytes > GROUP_SAMPLE_BYTES) return false;
-      if (k > g.first && sample + bytes > GROUP_SAMPLE_BYTES) break;
+      if (k > g.first && (sample + bytes > GROUP_SAMPLE_BYTES || k - g.first == GROUP_GRIDS))
+        break;
       G.mail = mail;
       G.sample = sample;
       mail += (long long)G.bands * 4 * G.strips * ROW_WORDS;

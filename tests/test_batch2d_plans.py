@@ -55,6 +55,14 @@ def test_waits_last_as_long_as_the_launch(adjoint):
     assert endless.wait_polls == 4_000_000_000  # bounded all the same
 
 
+# the monitors' kernels take a grid per blockIdx.y, which ends at 65535
+@pytest.mark.parametrize("n,launches,most", [(65535, 1, 65535), (65536, 2, 65535),
+                                             (140_000, 3, 65535)])
+def test_a_launch_takes_at_most_65535_grids(n, launches, most):
+    p = plan([(16, 32, 8)] * n, monitor=True)
+    assert (p.launches, p.most_grids) == (launches, most)
+
+
 def test_plans_reject_invalid_batches():
     cfg, arr = insts([(100, 100, 900)])
     out = _lib.DnBatch2dPlan()
