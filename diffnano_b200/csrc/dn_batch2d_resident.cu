@@ -32,7 +32,8 @@ struct Group {
 };
 constexpr int MAX_GROUPS = 256;
 struct Head {
-  int n_inst, n_cta, R, adjoint, n_groups, pad;
+  int n_inst, n_cta, R, adjoint, n_groups, dtype;
+  int curls, pad;  // curls: every grid has a curl record
   long long inst_offset, o_grids, bytes, ws_bytes;
   Group group[MAX_GROUPS];
 };
@@ -93,8 +94,11 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
   // slower turns (96 x 256^2, 2000 steps: 40 / 23 / 20 ms with R = 1 / 2 / 4; 12
   // recorded grids of 100^2 to 512^2: 3.9 / 3.2 / 3.9 ms, of 100^2 to 200^2 0.84 / 1.24 /
   // 3.3; their sweeps 5.5 / 5.3 and 1.3 / 2.2)
-  bool record = false;
-  for (int b = 0; b < n; ++b) record = record || insts[b].curl != nullptr;
+  bool record = false, curls = true;
+  for (int b = 0; b < n; ++b) {
+    record = record || insts[b].curl != nullptr;
+    curls = curls && insts[b].curl != nullptr;
+  }
   int R = 0;
   double best = 0.0;
   for (int r = 1; r <= (adjoint ? 2 : 4); r *= 2) {
@@ -118,6 +122,8 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
   h.n_cta = nsm;
   h.R = R;
   h.adjoint = adjoint;
+  h.curls = curls;
+  h.dtype = cfg->dtype;
   h.inst_offset = off;
   long long ws = 0;
   for (int k = 0; k < n;) {
@@ -174,6 +180,19 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
   }
   h.bytes = at;
   h.ws_bytes = ws;
+  return true;
+}
+
+// a batch as make_plan takes it; for a reverse sweep with all that the sweep reads and
+// writes
+bool valid(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint) {
+  if (!cfg || !insts || batch2d_inst_offset(cfg, insts) < 0) return false;
+  for (int b = 0; adjoint && b < cfg->n_inst; ++b) {
+    const dn_batch2d_inst& I = insts[b];
+    if (!I.curl || !I.grad) return false;
+    for (int c = 0; c < 3; ++c)
+      if (!I.lam[0][c] || !I.lam[1][c]) return false;
+  }
   return true;
 }
 
@@ -254,7 +273,7 @@ int run_groups(const Head& h, bool record, unsigned char* table, unsigned char* 
 
 extern "C" int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                              int32_t adjoint) {
-  if (!cfg || !insts) return -1;
+  if (!dn::res::valid(cfg, insts, adjoint != 0)) return -1;
   dn::res::Plan P;
   return dn::res::make_plan(cfg, insts, adjoint != 0, &P) ? P.h.bytes : 0;
 }
@@ -280,7 +299,7 @@ extern "C" int32_t dn_batch2d_resident_plan(const dn_batch2d* cfg, const dn_batc
 extern "C" int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                             int32_t adjoint, void* host_plan, int64_t bytes,
                                             int64_t* ws_bytes) {
-  if (!cfg || !insts || !host_plan || !ws_bytes) return DN_EINVAL;
+  if (!dn::res::valid(cfg, insts, adjoint != 0) || !host_plan || !ws_bytes) return DN_EINVAL;
   dn::res::Plan P;
   if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P)) return DN_EUNSUPPORTED;
   if (bytes < P.h.bytes) return DN_EINVAL;
@@ -306,7 +325,8 @@ extern "C" int32_t dn_batch2d_run_resident(const dn_batch2d* cfg, void* dev_tabl
         reinterpret_cast<uintptr_t>(ws)) & 15))
     return DN_EINVAL;
   const dn::res::Head& h = *static_cast<const dn::res::Head*>(host_plan);
-  if (cfg->n_inst != h.n_inst || cfg->pol != DN_TM || ws_bytes < h.ws_bytes || (h.ws_bytes && !ws))
+  if (cfg->n_inst != h.n_inst || cfg->pol != DN_TM || cfg->dtype != h.dtype ||
+      ws_bytes < h.ws_bytes || (h.ws_bytes && !ws) || (record && !h.adjoint && !h.curls))
     return DN_EINVAL;
   unsigned char *t = static_cast<unsigned char*>(dev_table),
                 *b = static_cast<unsigned char*>(dev_plan), *w = static_cast<unsigned char*>(ws);

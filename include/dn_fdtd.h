@@ -350,10 +350,12 @@ int32_t dn_batch2d_forward_cluster(const dn_batch2d* cfg, void* dev_table, int32
  * [n_steps][H*pitch]), and the reverse sweep (a plan made with adjoint = 1) reads
  * them, so it needs no replay.
  * dn_batch2d_resident_bytes: size of a plan, 0 when the batch has to go the other
- * way (TE, a grid that does not fit), -1 on invalid input.
+ * way (TE, a grid that does not fit), -1 on invalid input (a reverse sweep needs
+ * curl, grad and both lam sets of every grid).
  * dn_batch2d_resident_pack writes the plan into host memory; the caller copies it
  * to the device and passes both copies.  `ws`: device workspace of *ws_bytes
- * (contents irrelevant), 16-byte aligned; runs that share one must not overlap. */
+ * (contents irrelevant), 16-byte aligned; runs that share one must not overlap.
+ * `record` needs a plan whose grids all have curl (DN_EINVAL otherwise). */
 int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                   int32_t adjoint);
 int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,

@@ -74,6 +74,43 @@ def test_plans_reject_invalid_batches():
     assert call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out)) == _lib.DN_OK and out.rows == 0
 
 
+def test_a_reverse_sweep_needs_its_arrays():
+    size = _lib.lib().dn_batch2d_resident_bytes
+    cfg, arr = insts([(100, 100, 900)] * 2)
+    assert size(ctypes.byref(cfg), arr, 0) >= 0
+    for s in arr:
+        s.curl = s.grad = 16
+        for a in range(2):
+            for c in range(3):
+                s.lam[a][c] = 16
+    assert size(ctypes.byref(cfg), arr, 1) >= 0
+    arr[1].curl = None
+    assert size(ctypes.byref(cfg), arr, 1) == -1
+    arr[1].curl, arr[1].grad = 16, None
+    assert size(ctypes.byref(cfg), arr, 1) == -1
+    arr[1].grad, arr[1].lam[1][2] = 16, None
+    assert size(ctypes.byref(cfg), arr, 1) == -1
+    arr[0].H = 0
+    assert size(ctypes.byref(cfg), arr, 0) == -1
+
+
+@pytest.mark.gpu
+def test_a_recorded_run_needs_curl_records(cuda):
+    """A plan of grids without curl arrays refuses to record, and one of another type to
+    run (nothing is launched)."""
+    L = _lib.lib()
+    cfg, arr = insts([(64, 64, 20)] * 2)
+    n, ws = int(L.dn_batch2d_resident_bytes(ctypes.byref(cfg), arr, 0)), ctypes.c_int64(0)
+    assert n > 0
+    host = (ctypes.c_ubyte * n)()
+    _lib.check("pack", L.dn_batch2d_resident_pack(ctypes.byref(cfg), arr, 0, host, n,
+                                                  ctypes.byref(ws)))
+    run = L.dn_batch2d_run_resident
+    assert run(ctypes.byref(cfg), 16, host, 16, 16, 1 << 40, 1, None, None) == _lib.DN_EINVAL
+    cfg.dtype = _lib.DN_F64
+    assert run(ctypes.byref(cfg), 16, host, 16, 16, 1 << 40, 0, None, None) == _lib.DN_EINVAL
+
+
 @pytest.mark.gpu
 def test_a_band_waits_out_a_long_run_on_its_neighbours_cta(cuda):
     """One tiny grid of millions of steps on a CTA that a grid of a band per SM needs
