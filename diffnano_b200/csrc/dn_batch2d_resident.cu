@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <vector>
 
@@ -183,6 +184,17 @@ bool make_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint
   return true;
 }
 
+// f(), or `otherwise` where the host has no memory for a plan (no exception leaves a C
+// entry)
+template <typename R, typename F>
+R with_memory(R otherwise, const F& f) {
+  try {
+    return f();
+  } catch (const std::bad_alloc&) {
+    return otherwise;
+  }
+}
+
 // a batch as make_plan takes it; for a reverse sweep with all that the sweep reads and
 // writes
 bool valid(const dn_batch2d* cfg, const dn_batch2d_inst* insts, bool adjoint) {
@@ -274,8 +286,10 @@ int run_groups(const Head& h, bool record, unsigned char* table, unsigned char* 
 extern "C" int64_t dn_batch2d_resident_bytes(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                              int32_t adjoint) {
   if (!dn::res::valid(cfg, insts, adjoint != 0)) return -1;
-  dn::res::Plan P;
-  return dn::res::make_plan(cfg, insts, adjoint != 0, &P) ? P.h.bytes : 0;
+  return dn::res::with_memory<int64_t>(0, [&]() -> int64_t {
+    dn::res::Plan P;
+    return dn::res::make_plan(cfg, insts, adjoint != 0, &P) ? P.h.bytes : 0;
+  });
 }
 
 extern "C" int32_t dn_batch2d_resident_plan(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
@@ -283,37 +297,41 @@ extern "C" int32_t dn_batch2d_resident_plan(const dn_batch2d* cfg, const dn_batc
   if (!cfg || !insts || !out || n_sm < 0 || dn::batch2d_inst_offset(cfg, insts) < 0)
     return DN_EINVAL;
   *out = dn_batch2d_plan{};
-  dn::res::Plan P;
-  if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P, n_sm > 0 ? n_sm : dn::sm_count()))
+  return dn::res::with_memory<int32_t>(DN_ENOMEM, [&]() -> int32_t {
+    dn::res::Plan P;
+    if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P, n_sm > 0 ? n_sm : dn::sm_count()))
+      return DN_OK;
+    out->rows = P.h.R;
+    out->launches = P.h.n_groups;
+    for (int g = 0; g < P.h.n_groups; ++g) {
+      const dn::res::Group& G = P.h.group[g];
+      out->most_grids = std::max(out->most_grids, G.count);
+      out->wait_polls = std::max<int64_t>(out->wait_polls, dn::res::polls_of(G.steps));
+    }
     return DN_OK;
-  out->rows = P.h.R;
-  out->launches = P.h.n_groups;
-  for (int g = 0; g < P.h.n_groups; ++g) {
-    const dn::res::Group& G = P.h.group[g];
-    out->most_grids = std::max(out->most_grids, G.count);
-    out->wait_polls = std::max<int64_t>(out->wait_polls, dn::res::polls_of(G.steps));
-  }
-  return DN_OK;
+  });
 }
 
 extern "C" int32_t dn_batch2d_resident_pack(const dn_batch2d* cfg, const dn_batch2d_inst* insts,
                                             int32_t adjoint, void* host_plan, int64_t bytes,
                                             int64_t* ws_bytes) {
   if (!dn::res::valid(cfg, insts, adjoint != 0) || !host_plan || !ws_bytes) return DN_EINVAL;
-  dn::res::Plan P;
-  if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P)) return DN_EUNSUPPORTED;
-  if (bytes < P.h.bytes) return DN_EINVAL;
-  unsigned char* b = static_cast<unsigned char*>(host_plan);
-  std::memset(b, 0, (size_t)P.h.bytes);
-  std::memcpy(b, &P.h, sizeof(P.h));
-  std::memcpy(b + P.h.o_grids, P.grids.data(), P.grids.size() * sizeof(dn::res::ListGrid));
-  for (int g = 0; g < P.h.n_groups; ++g) {
-    std::memcpy(b + P.h.group[g].o_start, P.start[g].data(), P.start[g].size() * sizeof(int));
-    std::memcpy(b + P.h.group[g].o_jobs, P.jobs[g].data(),
-                P.jobs[g].size() * sizeof(dn::res::ListJob));
-  }
-  *ws_bytes = P.h.ws_bytes;
-  return DN_OK;
+  return dn::res::with_memory<int32_t>(DN_ENOMEM, [&]() -> int32_t {
+    dn::res::Plan P;
+    if (!dn::res::make_plan(cfg, insts, adjoint != 0, &P)) return DN_EUNSUPPORTED;
+    if (bytes < P.h.bytes) return DN_EINVAL;
+    unsigned char* b = static_cast<unsigned char*>(host_plan);
+    std::memset(b, 0, (size_t)P.h.bytes);
+    std::memcpy(b, &P.h, sizeof(P.h));
+    std::memcpy(b + P.h.o_grids, P.grids.data(), P.grids.size() * sizeof(dn::res::ListGrid));
+    for (int g = 0; g < P.h.n_groups; ++g) {
+      std::memcpy(b + P.h.group[g].o_start, P.start[g].data(), P.start[g].size() * sizeof(int));
+      std::memcpy(b + P.h.group[g].o_jobs, P.jobs[g].data(),
+                  P.jobs[g].size() * sizeof(dn::res::ListJob));
+    }
+    *ws_bytes = P.h.ws_bytes;
+    return DN_OK;
+  });
 }
 
 extern "C" int32_t dn_batch2d_run_resident(const dn_batch2d* cfg, void* dev_table,

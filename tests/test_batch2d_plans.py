@@ -4,6 +4,9 @@ and the batches that a plan must not break."""
 from __future__ import annotations
 
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -72,6 +75,31 @@ def test_plans_reject_invalid_batches():
     assert call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out)) == _lib.DN_EINVAL
     cfg.pol, arr[0].H = _lib.DN_TE, 100
     assert call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out)) == _lib.DN_OK and out.rows == 0
+
+
+NO_MEMORY = """
+import ctypes, resource, sys
+sys.path.insert(0, sys.argv[1])
+from test_batch2d_plans import SMS, _lib, insts
+cfg, arr = insts([(16, 32, 8)] * 300_000)
+out, call = _lib.DnBatch2dPlan(), _lib.lib().dn_batch2d_resident_plan
+used = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+limit = resource.getrlimit(resource.RLIMIT_AS)
+resource.setrlimit(resource.RLIMIT_AS, (used + (1 << 20), limit[1]))
+rc = call(ctypes.byref(cfg), arr, 0, SMS, ctypes.byref(out))
+resource.setrlimit(resource.RLIMIT_AS, limit)
+print(rc, out.rows)
+"""
+
+
+def test_a_host_without_memory_for_a_plan_gets_a_status():
+    """(in a process of its own: its address space ends 1 MB further on)"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    r = subprocess.run([sys.executable, "-c", NO_MEMORY, here], capture_output=True, text=True,
+                       timeout=300, cwd=os.path.dirname(here),
+                       env={**os.environ, "PYTHONPATH": os.path.dirname(here)})
+    assert r.returncode == 0, r.stderr
+    assert r.stdout.split() == [str(_lib.DN_ENOMEM), "0"]
 
 
 def test_a_reverse_sweep_needs_its_arrays():
