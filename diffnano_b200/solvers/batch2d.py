@@ -222,6 +222,7 @@ class FDTDBatch2D:
         self.K = int(checkpoint_interval or max(1, math.ceil(math.sqrt(T))))
         self.tile_rows = tile_rows
         self._auto_rows = tile_rows is None
+        self._tuned_rows = None  # what autotune_tile_rows chose
         self._asked_checkpoints = checkpoint_interval is not None
         self._record = None  # room for the curl terms of all steps, or None
         self._plans: dict = {}  # adjoint? -> (host plan, device plan, workspace bytes)
@@ -261,14 +262,14 @@ class FDTDBatch2D:
         self._grad_alloc = grad
         self._graph = None
         if self._auto_rows:
-            self.tile_rows = 16
+            self.tile_rows = self._tuned_rows or 16
         if grad or not self.cluster:
             self._plan_resident()
         if self._record is not None and (False not in self._plans or True not in self._plans):
             self._record = self._insts = None  # some grid does not fit on the chip
             self._make_insts(grad, views, record=False)
-        if self._auto_rows and not self.uses_resident(True, grad):
-            self.tile_rows = autotune_tile_rows(self)
+        if self._auto_rows and not self._tuned_rows and not self.uses_resident(True, grad):
+            self.tile_rows = self._tuned_rows = autotune_tile_rows(self)
         self._pack()
 
     def _make_insts(self, grad: bool, views, record: bool) -> None:

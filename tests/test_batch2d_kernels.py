@@ -4,11 +4,14 @@ against the CPU FP64 oracle."""
 
 from __future__ import annotations
 
+from dataclasses import replace
+
 import pytest
 import torch
 from conftest import rel_l2
 
 from diffnano_b200 import _lib
+from diffnano_b200.solvers import batch2d
 from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D
 from oracle import fdtd_ref as R
 
@@ -92,3 +95,19 @@ def test_a_graph_replay_keeps_the_cluster_kernel(cuda, monkeypatch):
     replayed, _ = b.forward_graphed(eps)
     assert ran == "dn_batch2d_forward_cluster"
     assert all(torch.equal(x, y) for x, y in zip(fields, replayed))
+
+
+@pytest.mark.gpu
+def test_tile_heights_are_timed_once(cuda, monkeypatch):
+    """A batch that alternates between solves with and without gradient keeps the tile
+    height it has chosen."""
+    calls = []
+    monkeypatch.setattr(batch2d, "autotune_tile_rows", lambda b: calls.append(1) or 32)
+    eps = [e.to(cuda) for e in _eps()]
+    b = FDTDBatch2D([replace(s, monitor=None) for s in _specs()], "TE", torch.float64, cuda)
+    for _ in range(2):
+        b.forward(eps)
+        fields, _ = b.forward([e.requires_grad_(True) for e in eps])
+        torch.autograd.grad(sum(f.sum() for f in fields), eps)
+        eps = [e.detach() for e in eps]
+    assert len(calls) == 1 and b.tile_rows == 32
