@@ -142,7 +142,7 @@ __device__ __forceinline__ void filter_tile(const Taps& taps, int H, int W, int 
 __global__ void __launch_bounds__(NTF)
     k_density_fwd(const float* __restrict__ rho, int nl, int H, int W, int kind, float beta,
                   float eta, float den, float off, float lo, float span,
-                  float* __restrict__ filtered, float* __restrict__ eps,
+                  float* filtered, float* eps,  // (may be one buffer: eps is what stays)
                   const __grid_constant__ Taps taps) {
   const int nx = (W + TW - 1) / TW;
   const int h0 = blockIdx.x / nx * TH, w0 = blockIdx.x % nx * TW;
@@ -312,12 +312,13 @@ void proj_consts(const dn_density* d, float* den, float* off) {
   *den = *off + tanhf(d->beta * (1.0f - d->eta));
 }
 
-// A tile reads its neighbours' cells, so an input that is also an output is read
-// from a copy in `work`.
+// A tile reads its neighbours' cells, so an input that shares memory with an output is
+// read from a copy in `work`.
 int apart(const dn_density* d, const float** in, const float* out, float* work, cudaStream_t s) {
-  if (*in != out) return DN_OK;
-  DN_CUDA_CHECK(cudaMemcpyAsync(work, *in, (size_t)d->n_layers * d->H * d->W * sizeof(float),
-                                cudaMemcpyDeviceToDevice, s));
+  const size_t bytes = (size_t)d->n_layers * d->H * d->W * sizeof(float);
+  const uintptr_t a = reinterpret_cast<uintptr_t>(*in), b = reinterpret_cast<uintptr_t>(out);
+  if (a + bytes <= b || b + bytes <= a) return DN_OK;
+  DN_CUDA_CHECK(cudaMemcpyAsync(work, *in, bytes, cudaMemcpyDeviceToDevice, s));
   *in = work;
   return DN_OK;
 }

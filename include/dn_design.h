@@ -45,7 +45,8 @@ typedef struct dn_density {
 
 /* filtered = filter(rho); eps = lo + (hi - lo) * project(filtered).  work,
  * filtered and eps each hold n_layers*H*W floats; keep `filtered` for the
- * backward pass.  An output may be the input's buffer (work then holds a copy). */
+ * backward pass.  Outputs may share memory with the input (work then holds a
+ * copy of it). */
 int32_t dn_density_forward(const dn_density* d, const float* rho, float* work, float* filtered,
                            float* eps, void* stream);
 /* drho = filter(d eps * (hi - lo) * project'(filtered)); work as above. */

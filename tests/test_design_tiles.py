@@ -64,6 +64,38 @@ def test_density_outputs_may_be_the_input(cuda):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shift", [1, 149, 70 * 150, 2 * 70 * 150 - 1])
+def test_density_outputs_may_share_memory_with_the_input(cuda, shift):
+    """Outputs that begin `shift` values into the input, or before it, and one buffer
+    for both outputs (eps is what stays)."""
+    import ctypes
+
+    from diffnano_b200 import _lib
+    g = torch.Generator().manual_seed(6)
+    rho = torch.rand(2, 70, 150, generator=g).to(cuda)
+    n = rho.numel()
+    d = _lib.DnDensity(2, 70, 150, 1, 3.0, 4.0, 0.5, 1.0, 3.0)
+    work, filt, eps, other = (torch.empty_like(rho) for _ in range(4))
+    s = torch.cuda.current_stream().cuda_stream
+
+    def run(r, f, e):
+        assert _lib.lib().dn_density_forward(ctypes.byref(d), r.data_ptr(), work.data_ptr(),
+                                             f.data_ptr(), e.data_ptr(), s) == 0
+
+    run(rho, filt, eps)
+    for first, second in ((0, shift), (shift, 0)):
+        for swap in (False, True):
+            buf = torch.zeros(n + shift, device=cuda)
+            r, o = buf[first:first + n], buf[second:second + n]
+            r.copy_(rho.reshape(-1))
+            run(r, *((other, o) if swap else (o, other)))
+            want = (filt, eps) if swap else (eps, filt)
+            assert torch.equal(other, want[0]) and torch.equal(o, want[1].reshape(-1))
+    run(rho, other, other)
+    assert torch.equal(other, eps)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(1, 1, 1), (2, 8, 32), (3, 9, 33), (1, 1, 70), (2, 70, 1)])
 def test_blocks_of_the_pools(cuda, shape):
     from diffnano_b200.design import projection as P
