@@ -14,6 +14,7 @@ from conftest import rel_l2
 
 from diffnano_b200 import _lib
 from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D
+from oracle import fdtd_ref as R
 
 SMS = 148
 SPIN_LIMIT, POLLS_PER_STEP = 1 << 22, 64
@@ -120,6 +121,36 @@ def test_a_reverse_sweep_needs_its_arrays():
     assert size(ctypes.byref(cfg), arr, 1) == -1
     arr[0].H = 0
     assert size(ctypes.byref(cfg), arr, 0) == -1
+
+
+def _rows(specs, dtype, curl=False, adjoint=False):
+    cfg, arr = insts([(*s.grid_shape, s.n_steps) for s in specs])
+    cfg.dtype = _lib.DN_F32 if dtype == torch.float32 else _lib.DN_F64
+    for s in arr:
+        s.curl = 16 if curl else None
+    out = _lib.DnBatch2dPlan()
+    _lib.check("plan", _lib.lib().dn_batch2d_resident_plan(ctypes.byref(cfg), arr, int(adjoint), SMS,
+                                                           ctypes.byref(out)))
+    return out.rows
+
+
+# the two batches of tests/test_batch2d_resident.py run with 1 and 4 rows per warp and
+# sweep with 1 and 2; here the runs with two rows
+@pytest.mark.gpu
+@pytest.mark.parametrize("shapes,dtype", [([(300, 413)] * 3, torch.float32),
+                                          ([(300, 400), (200, 129)], torch.float64)])
+def test_a_batch_with_two_rows_per_warp(cuda, shapes, dtype):
+    specs = [BatchInstance(grid_shape=s, n_steps=24 + 6 * (s[0] < 300), pml_layers=4,
+                           source={"type": "gaussian_pulse", "row": 20, "spread": 100.0, "t0": 80.0})
+             for s in shapes]
+    assert _rows(specs, dtype) == 2
+    g = torch.Generator().manual_seed(7)
+    eps = [(1.5 + 2.0 * torch.rand(*s, dtype=torch.float64, generator=g)).to(cuda) for s in shapes]
+    fields, _ = FDTDBatch2D(specs, "TM", dtype, cuda, tile_rows=16).forward(eps)
+    for spec, e, f in zip(specs, eps, fields):
+        o = R.run_2d(e.cpu(), dl=spec.dl, dt=spec.dt, omega=spec.omega, pml_layers=4,
+                     n_steps=spec.n_steps, source=spec.source)
+        assert rel_l2(f, o["Ez"]) < (1e-5 if dtype == torch.float32 else 1e-12)
 
 
 @pytest.mark.gpu

@@ -8,12 +8,13 @@ import ctypes
 import pytest
 import torch
 from conftest import rel_l2
-from test_resident2d import _compare, _comps, _engine, _sweep, _tol
+from test_resident2d import _compare, _compare_sweeps, _comps, _engine, _run, _sweep, _tol
 from test_resident3d import _compare as _compare3d
 from test_resident3d import _engine as _engine3d
 
 from diffnano_b200 import _lib
 from diffnano_b200.solvers._engine import MonitorSpec
+from oracle import fdtd_ref as R
 
 SMS = 148
 TM, TE, F32, F64 = _lib.DN_TM, _lib.DN_TE, torch.float32, torch.float64
@@ -120,3 +121,63 @@ def test_a_3d_step_more_than_a_launch_holds(cuda):
     T = (64 << 20) // (48 ** 3 * 4) + 1
     mons = [MonitorSpec("a", _lib.DN_EY, tuple((0, n) for n in shape), (1550.0,))]
     _compare3d(_engine3d(shape, _lib.DN_AXES_PHYSICAL, T, {"pos": [20, 20, 20]}, monitors=mons))
+
+
+# (shape, rows per warp of a run / of a reverse sweep), FP32 TM: one cluster up to 16
+# bands, then the fewest rows for which a band per SM holds the grid
+PLANS_F32 = [((1, 1), 1, 1), ((100, 100), 1, 1), ((256, 256), 2, 2), ((257, 256), 1, 1),
+             ((300, 413), 1, 1), ((598, 513), 2, 2), ((701, 701), 3, 3), ((1023, 1021), 4, 0),
+             ((1200, 1000), 0, 0), ((16, 2048), 2, 2), ((16, 2049), 0, 0)]
+PLANS_F64 = [((100, 100), 2, 2), ((333, 270), 1, 1), ((601, 499), 3, 3), ((1100, 450), 4, 0),
+             ((598, 513), 0, 0), ((16, 1024), 2, 2), ((16, 1025), 0, 0)]
+
+
+@pytest.mark.parametrize("dtype,plans", [(F32, PLANS_F32), (F64, PLANS_F64)])
+def test_rows_per_warp(dtype, plans):
+    for (H, W), run, sweep in plans:
+        assert plan2d(H, W, 100, TM, dtype).rows == run
+        assert plan2d(H, W, 100, TM, dtype, adjoint=True).rows == sweep
+        assert plan2d(H, W, 100, TE, dtype).rows == (run if dtype == F64 else 0)
+        assert plan2d(H, W, 100, TE, dtype, adjoint=True).rows == 0
+        assert plan2d(H, W, 7, TM, dtype).rows == 0
+    assert plan2d(256, 256, 100).cluster and not plan2d(257, 256, 100).cluster
+
+
+# blocks of three and four rows, the last band and the last block ragged
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,W,pol,dtype,rows", [
+    (701, 701, TM, F32, 3), (1023, 1021, TM, F32, 4), (601, 499, TM, F64, 3), (601, 499, TE, F64, 3),
+    (1100, 450, TM, F64, 4), (1099, 449, TE, F64, 4)])
+def test_blocks_of_more_rows(cuda, H, W, pol, dtype, rows):
+    assert plan2d(H, W, 9, pol, dtype).rows == rows
+    for T in (9, 24):
+        f = _lib.DN_EZ if pol == TM else _lib.DN_HZ
+        _compare(_engine(H, W, pol, dtype, T, [MonitorSpec("box", f, ((0, 1), (H // 2, H // 2 + 5),
+                                                                     (3, W - 2)), [1550.0])]), pol, T)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,W,dtype", [(701, 701, F32), (601, 499, F64)])
+def test_reverse_sweep_of_blocks_of_three_rows(cuda, H, W, dtype):
+    assert plan2d(H, W, 9, TM, dtype, adjoint=True).rows == 3
+    f = _lib.DN_EZ
+    _compare_sweeps(cuda, H, W, dtype, [
+        MonitorSpec("row", f, ((0, 1), (H // 2, H // 2 + 1), (0, W)), [1500.0, 1600.0]),
+        MonitorSpec("box", f, ((0, 1), (0, (H + 1) // 2), (W // 2, W)), [1550.0])])
+
+
+# (solves of this size run resident, so the kernel is called by its own entry point)
+@pytest.mark.gpu
+@pytest.mark.parametrize("pol,comp", [(TM, "Ez"), (TE, "Hz")])
+def test_launch_by_launch_kernel_on_a_large_grid_against_the_oracle(cuda, pol, comp):
+    n, T = 1024, 30
+    g = torch.Generator().manual_seed(n * 1000 + n)
+    eps = 1.5 + 2.0 * torch.rand(n, n, dtype=F64, generator=g)  # as _engine makes it
+    eng = _engine(n, n, pol, F32, T)
+    eng.reset()
+    _run(eng, False, 0, T)
+    src = {"type": "gaussian_pulse", "row": n // 3, "spread": 300.0, "t0": 700.0}
+    o = R.run_2d(eps, dl=20.0, dt=eng.dt, omega=2 * 3.14159 / 1550.0, pml_layers=4,
+                 polarization="TM" if pol == TM else "TE", n_steps=T, source=src)
+    assert float(o[comp].abs().max()) > 0
+    assert rel_l2(eng.field(_lib.COMPONENTS[comp])[0], o[comp]) < 1e-5
