@@ -62,21 +62,6 @@ def padded_width(W: int) -> int:
     return (W + 31) // 32 * 32
 
 
-def runs_resident_2d(shape, dtype: torch.dtype, pol: int, n_steps: int, device) -> bool:
-    """Whether a 2-D run keeps its fields on the chip (monitors of a grid that could do
-    without this never change the answer: their samples are far below the workspace's
-    share)."""
-    H, W = (int(v) for v in shape)
-    Wp = padded_width(W)
-    grid = _lib.DnGrid(D=1, H=H, W=W, dtype=_lib.DN_F32 if dtype == torch.float32 else _lib.DN_F64,
-                       pitch_y=Wp, pitch_z=H * Wp, dt=1.0, dl=1.0, axes=0, pol=pol)
-    plan = _lib.DnResidentPlan()
-    with torch.cuda.device(device):
-        rc = _lib.lib().dn_fdtd2d_resident_plan(ctypes.byref(grid), None, None, 0, int(n_steps), 0,
-                                                0, ctypes.byref(plan))
-    return rc == _lib.DN_OK and plan.rows > 0
-
-
 @dataclass
 class MonitorSpec:
     name: str

@@ -28,18 +28,16 @@ from diffnano_b200.solvers._common import (
     monitor_metadata,
     parse_monitors,
 )
-from diffnano_b200.solvers._engine import (
-    Engine,
-    compute_device,
-    runs_resident_2d,
-    to_result_device,
-)
+from diffnano_b200.solvers._engine import Engine, compute_device, to_result_device
 from diffnano_b200.solvers._result import SimResult
 
 __all__ = ["FDTDSolver2D"]
 
 _TM_FIELDS = ("Ez", "Hx", "Hy")
 _TE_FIELDS = ("Hz", "Ex", "Ey")
+# Shorter runs do not run resident, nor does FP32 TE.  (Of the other grids that do not,
+# none is one for the cluster kernel: their rows or columns are too long for it.)
+_MIN_RESIDENT_STEPS = 8
 
 
 class FDTDSolver2D:
@@ -127,7 +125,9 @@ class FDTDSolver2D:
         probe = src.get("probe", None)
         needs_grad = torch.is_grad_enabled() and eps.requires_grad
         fast = None
-        if probe is None and not needs_grad and not self._resident():
+        if probe is None and not needs_grad and (self.n_steps < _MIN_RESIDENT_STEPS or
+                                                 (self.polarization == "TE" and
+                                                  self.dtype == torch.float32)):
             fast = self._cluster_solve(eps, src, mons)
         if fast is not None:
             specs, field, dfts = fast
@@ -176,18 +176,6 @@ class FDTDSolver2D:
                 cache.clear()
             cache[key] = make()
         return cache[key]
-
-    def _resident(self) -> bool:
-        """Whether a solve of this set-up runs resident."""
-        key = (tuple(self.grid_shape), self.dtype, self.polarization, self.n_steps,
-               str(self._device))
-        known = self.__dict__.setdefault("_resident_known", {})
-        if key not in known:
-            known.clear()
-            known[key] = runs_resident_2d(self.grid_shape, self.dtype,
-                                          _lib.DN_TM if self.polarization == "TM" else _lib.DN_TE,
-                                          self.n_steps, compute_device(self._device))
-        return known[key]
 
     def _cluster_solve(self, eps, src, mons):
         """Gradient-free solve with the whole grid in one thread-block cluster

@@ -4,6 +4,7 @@ launch where the grid fits a thread-block cluster and its warps have little to w
 from __future__ import annotations
 
 import pytest
+import test_resident_plans as plans
 import torch
 from conftest import rel_l2
 from test_batch2d_kernels import _Recorder
@@ -24,6 +25,18 @@ def test_what_fits_a_cluster():
     assert not fits(1024, 1024) and not fits(700, 700, "TM", F64) and not fits(64, 64, T=0)
     assert fits(64, 64, mon={"row": 3, "wavelengths_nm": [1550.0]})
     assert not fits(64, 64, mon={"row": 3, "wavelengths_nm": []})
+
+
+def test_no_other_grid_is_one_for_the_cluster():
+    """What FDTDSolver2D takes for granted: beside FP32 TE and runs of under 8 steps, no
+    grid within the cluster rule's 24 pieces lacks a resident plan."""
+    for pol, dtype in ((plans.TM, F32), (plans.TM, F64), (plans.TE, F64)):
+        assert plans.plan2d(100, 100, 8, pol, dtype).rows > 0
+        assert plans.plan2d(100, 100, 7, pol, dtype).rows == 0
+        for pieces in range(1, 25):
+            for turns in range(1, 24 // pieces + 1):
+                H, W = 256 * turns, 32 * pieces
+                assert plans.plan2d(H, W, 8, pol, dtype).rows > 0
 
 
 def _forward(monkeypatch, solver, *a, **kw):
