@@ -19,11 +19,11 @@
 namespace dn {
 namespace res {
 
-template <typename T, int R, int MAIL>
+template <typename T, int R, int MAIL, bool LISTED>
 __device__ __forceinline__ void sweep_band(const AdjJob<T>& J, const Split& S, int band,
                                            unsigned char* smem, uint64_t* mail, unsigned polls,
                                            int* status, const Samples<T>* adds, int n_add) {
-  using B = Block<T, R, MAIL>;
+  using B = Block<T, R, MAIL, LISTED>;
   using L = typename B::L;
   constexpr int VEC = B::VEC;
   constexpr int COLS = B::COLS;
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   if constexpr (MAIL == MAIL_CLUSTER) arm_mailboxes<L>(r_smem);
   const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
   if (!skip && (int)blockIdx.x < S.bands)
-    sweep_band<T, R, MAIL>(J, S, blockIdx.x, r_smem, mail, SPIN_LIMIT, status, adds.s, adds.n);
+    sweep_band<T, R, MAIL, false>(J, S, blockIdx.x, r_smem, mail, 0, status, adds.s, adds.n);
   if constexpr (MAIL == MAIL_CLUSTER) cg::this_cluster().sync();  // no row still under way
 }
 

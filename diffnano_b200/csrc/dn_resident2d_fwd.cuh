@@ -10,11 +10,11 @@ namespace res {
 // ---------------------------------------------------------------------------
 // the run of one band
 // ---------------------------------------------------------------------------
-template <typename T, int POL, int R, int MAIL, bool REC, bool SMP>
+template <typename T, int POL, int R, int MAIL, bool REC, bool SMP, bool LISTED>
 __device__ __forceinline__ void run_band(const Job<T>& J, const Split& S, int band,
                                          unsigned char* smem, uint64_t* mail, unsigned polls,
                                          int* status, const Samples<T>* smps, int n_smp) {
-  using B = Block<T, R, MAIL>;
+  using B = Block<T, R, MAIL, LISTED>;
   using L = typename B::L;
   constexpr int VEC = B::VEC;
   constexpr int COLS = B::COLS;
@@ -267,8 +267,8 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
   // a previous launch that recorded an error turns this one into a no-op
   const bool skip = status != nullptr && *reinterpret_cast<const volatile int*>(status) != 0;
   if (!skip && (int)blockIdx.x < S.bands)
-    run_band<T, POL, R, MAIL, REC, SMP>(J, S, blockIdx.x, r_smem, mail, SPIN_LIMIT, status,
-                                             smps.s, smps.n);
+    run_band<T, POL, R, MAIL, REC, SMP, false>(J, S, blockIdx.x, r_smem, mail, 0, status, smps.s,
+                                               smps.n);
   if constexpr (MAIL == MAIL_CLUSTER) cg::this_cluster().sync();  // no row still under way
 }
 

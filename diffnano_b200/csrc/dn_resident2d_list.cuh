@@ -73,11 +73,12 @@ __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
     __syncthreads();
     const int n = I.mon_comp != DN_NONE && (!ADJ || I.gmon != nullptr);
     if constexpr (ADJ)
-      sweep_band<T, R, MAIL_GLOBAL>(A, S, job.band, r_smem, L.mail + G.mail, L.polls, status, &smp,
-                                    n);
+      sweep_band<T, R, MAIL_GLOBAL, true>(A, S, job.band, r_smem, L.mail + G.mail, L.polls,
+                                          status, &smp, n);
     else
-      run_band<T, DN_TM, R, MAIL_GLOBAL, REC, true>(J, S, job.band, r_smem, L.mail + G.mail,
-                                                   L.polls, status, &smp, n);
+      run_band<T, DN_TM, R, MAIL_GLOBAL, REC, true, true>(J, S, job.band, r_smem,
+                                                          L.mail + G.mail, L.polls, status, &smp,
+                                                          n);
   }
 }
 
