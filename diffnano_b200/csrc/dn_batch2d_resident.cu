@@ -48,8 +48,8 @@ struct Plan {
 
 inline long long up16(long long x) { return (x + 15) / 16 * 16; }
 
-// us per step of bands with R = 1, 2, 4 rows per warp (B200, FP32, 16 warps): run,
-// recorded run, reverse sweep
+// us per step of bands with R = 1, 2, 4 rows per warp (B200, FP32, 16 warps; FP64 goes
+// by the same, unmeasured): run, recorded run, reverse sweep
 constexpr double STEP_US[3][3] = {{0.82, 1.06, 1.66}, {1.0, 1.5, 4.0}, {1.4, 2.6, 0.0}};
 
 // The CTAs by the steps they have been given, fewest first.

@@ -690,7 +690,8 @@ int launch_all(const StepParams<T>& base, const TmapSet& ta, const TmapSet& tb, 
   // planes of the step before are marched (2.5 us of each step on B200; released from
   // its first plane on, a step's CTAs spread unevenly over the SMs behind the running
   // ones, and 256^3 lost 5 %).  Steps that write a curl record on large grids do without:
-  // 192^3 99 -> 95 us per step with them, 256^3 206 -> 213.
+  // 192^3 99 -> 95 us per step with them, 256^3 206 -> 213 (no other size was measured;
+  // the line lies between these two).
   const bool chain = !REC || (long long)base.D * base.H * base.W <= 1LL << 23;
   for (int n = 0; n < nsteps; ++n) {
     const bool even = (n % 2) == 0;

@@ -20,7 +20,9 @@ namespace {
 // 0.95 (R = 1), 1.0 - 1.2 (R = 2), 1.6 - 2.0 (R = 3), 1.9 - 2.2 (R = 4), where
 // one launch per step takes 6.2 (256 x 256) to 8.3 (1024 x 1024).  So: a cluster
 // where 16 bands hold the grid, else the fewest rows per warp for which one
-// band per SM does.  The reverse sweep holds the FP64 gradient too: at most
+// band per SM does.  (At 16 warps of two rows, about 192^2 to 256^2 in FP32, the
+// cluster's 0.76 and the whole chip's 0.7 - 0.95 have not been compared on one grid;
+// FP64 goes by the FP32 figures.)  The reverse sweep holds the FP64 gradient too: at most
 // R = 3 (909 k cells in FP32).
 constexpr int R_MAX = 4, R_MAX_ADJ = 3;
 Split choose_split(int H, int W, int elem, int nsm, int r_max) {

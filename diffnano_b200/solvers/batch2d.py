@@ -1,22 +1,21 @@
-"""Batched 2-D FDTD: many independent grids in one persistent launch.
+"""Batched 2-D FDTD: many independent grids at once.
 
 The reference solves one grid per ``FDTDSolver2D`` object with a Python step
 loop (``diffnano/solvers/fdtd2d.py:309-357``).  Design studies need many small
 to medium grids at once -- robust erosion/dilation variants of a design,
-wavelength sweeps -- of different sizes and step counts.  ``FDTDBatch2D``
-advances all of them in one persistent cooperative kernel
-(``dn_batch2d_forward``) and differentiates all of them in a second one
-(``dn_batch2d_backward``: checkpoint-segment replay + reverse steps), with the
-same step arithmetic as the single-grid kernels.  TM batches whose grids fit on
-the chip run grid by grid with the fields in registers instead
-(``dn_batch2d_run_resident``): always without a gradient, and with one where there
-is room for the curl terms of all steps (``_records``; and no
-``checkpoint_interval`` was asked for).  Each instance is described
-by the reference's own constructor arguments and source dict, plus one DFT
-line/point/box monitor on its injected field.
+wavelength sweeps -- of different sizes and step counts.  TM batches whose grids
+fit on the chip run grid by grid with the fields in registers
+(``dn_batch2d_run_resident``): always without a gradient (unless ``cluster=True``),
+and with one where there is room for the curl terms of all steps (``_records``;
+and no ``checkpoint_interval`` was asked for).  The others are advanced by one
+persistent cooperative kernel (``dn_batch2d_forward``) and differentiated by a
+second one (``dn_batch2d_backward``: checkpoint-segment replay + reverse steps),
+with the same step arithmetic as the single-grid kernels.  Each instance is
+described by the reference's own constructor arguments and source dict, plus one
+DFT line/point/box monitor on its injected field.
 
 ``forward`` is differentiable with respect to every instance's eps;
-``forward_graphed`` records the eps upload, reset and persistent launch in a
+``forward_graphed`` records the eps upload, reset and launches in a
 CUDA graph and replays it when the same batch is solved repeatedly (design
 iterations).  The tile height is
 chosen by ``autotune_tile_rows`` (measured, cached per device and batch
@@ -188,7 +187,7 @@ def _cache_path() -> str:
 
 
 class FDTDBatch2D:
-    """Many 2-D grids (same polarisation) solved by one persistent launch.
+    """Many 2-D grids (same polarisation) solved together.
 
     Parameters
     ----------
@@ -458,7 +457,7 @@ class FDTDBatch2D:
 
     def forward_graphed(self, eps_list):
         """``run_forward`` through a CUDA graph: the first call records the
-        eps upload, state reset and persistent launch; later calls copy the
+        eps upload, state reset and launches; later calls copy the
         new eps into the recorded input buffers and replay.  No autograd."""
         self._build(False)
         if self._graph is None:

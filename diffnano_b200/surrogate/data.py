@@ -4,8 +4,8 @@ Designs are seeded binary Si/SiO2 blob maps (N(0,1) noise, Gaussian filter of
 sigma drawn from [2, 6] cells, threshold 0 -- the blob recipe of the 256x256
 TMz workload) placed in the central 128x128 region of a 256x256 SiO2 grid.
 Each design is labelled with the complex DFT of Ez on the central 128 cells of
-the monitor row at three wavelengths, computed by ``FDTDBatch2D`` (one
-persistent launch per chunk of designs) with the workload's set-up: dx = 20
+the monitor row at three wavelengths, computed by ``FDTDBatch2D`` (a
+resident run per chunk of designs) with the workload's set-up: dx = 20
 nm, 20-cell CPML, Courant 0.5, 2000 steps, Gaussian-pulse line source at row
 30 (1.55 um centre, 0.2 um width), monitor row 226 at 1.50 / 1.55 / 1.60 um.
 """
@@ -91,7 +91,7 @@ def design_eps(masks: torch.Tensor) -> torch.Tensor:
 
 class FDTDLabeler:
     """Labels design-region permittivity maps with monitor DFTs by running the
-    batched FDTD on chunks of ``chunk`` designs (one persistent launch each)."""
+    batched FDTD on chunks of ``chunk`` designs."""
 
     def __init__(self, setup: TMzSetup = TMzSetup(), chunk: int = 2048, device="cuda"):
         self.setup = setup
@@ -103,6 +103,8 @@ class FDTDLabeler:
 
     def _solver(self, n: int) -> FDTDBatch2D:
         if self._batch is None or self._n != n:
+            # (the last two count only where a resident run finds no workspace: such a chunk
+            # streams faster through 32-row tiles than one cluster per grid)
             self._batch = FDTDBatch2D([self.setup.instance() for _ in range(n)], "TM",
                                       torch.float32, self.device, tile_rows=32, cluster=False)
             self._n = n
