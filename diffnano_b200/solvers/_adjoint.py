@@ -58,7 +58,7 @@ class _Runner:
         eng.reset()
         eng.set_eps(eps_dev)
         T, K = eng.n_steps, self.K
-        if save and self.full_record:
+        if save and self.full_record and T > 0:
             # beside it: two adjoint states, the FP64 gradient, the outputs
             beside = 3 * eng.A.nbytes + 8 * eng.ce.numel()
             self.record = _records.claim(eng.device, eng.curl_bytes(T), beside,

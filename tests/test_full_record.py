@@ -54,3 +54,16 @@ def test_checkpoints_when_the_record_does_not_fit(cuda, monkeypatch):
     f1, g1 = _gradient(_solver3d(cuda), eps, src)
     assert asked[0] == 37 and 0 < asked[1] < 37
     assert torch.equal(f0, f1) and torch.equal(g0, g1)
+
+
+@pytest.mark.parametrize("make", [
+    lambda dev: dn.FDTDSolver2D(grid_shape=(20, 30), pml_layers=4, n_steps=0, device=dev),
+    lambda dev: dn.FDTDSolver2D(grid_shape=(20, 30), polarization="TE", n_steps=0, device=dev),
+    lambda dev: dn.FDTDSolver3D(grid_shape=(8, 9, 10), pml_layers=2, n_steps=0, device=dev,
+                                cpml_axes="physical")], ids=["tm", "te", "3d"])
+def test_a_solve_without_steps_has_a_gradient_of_zero(cuda, make):
+    s = make(cuda)
+    e = torch.full(s.grid_shape, 2.0, dtype=torch.float64, device=cuda, requires_grad=True)
+    r = s.forward(e, source={"type": "gaussian_pulse"})
+    (g,) = torch.autograd.grad((r.field.double() ** 2).sum() + r.field.sum(), e)
+    assert not r.field.any() and g.shape == e.shape and not g.any()
