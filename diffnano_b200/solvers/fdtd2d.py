@@ -4,8 +4,8 @@ Same constructor, attributes, ``forward`` and ``time_series`` as the
 reference (``diffnano/solvers/fdtd2d.py:91-524``); every time step runs in the
 CUDA kernels behind ``dn_fdtd2d_run_ws`` (``include/dn_fdtd.h``): grids that fit on
 the chip take all steps in one launch, larger ones one launch per step; solves without
-gradient that it would step launch by launch (FP32 TE, a few steps) run in one
-thread-block cluster where that is faster.  Additions, all
+gradient that are short, or in FP32 TE (which it would step launch by launch), run in
+one thread-block cluster where that is faster.  Additions, all
 optional keyword arguments: ``backward`` ("auto"/"autograd"/"time_reversal"/
 "checkpoint"), ``dtype`` (torch.float32 default, torch.float64 for
 validation), and DFT ``monitors``.
@@ -35,9 +35,6 @@ __all__ = ["FDTDSolver2D"]
 
 _TM_FIELDS = ("Ez", "Hx", "Hy")
 _TE_FIELDS = ("Hz", "Ex", "Ey")
-# Shorter runs do not run resident, nor does FP32 TE.  (Of the other grids that do not,
-# none is one for the cluster kernel: their rows or columns are too long for it.)
-_MIN_RESIDENT_STEPS = 8
 
 
 class FDTDSolver2D:
@@ -125,9 +122,7 @@ class FDTDSolver2D:
         probe = src.get("probe", None)
         needs_grad = torch.is_grad_enabled() and eps.requires_grad
         fast = None
-        if probe is None and not needs_grad and (self.n_steps < _MIN_RESIDENT_STEPS or
-                                                 (self.polarization == "TE" and
-                                                  self.dtype == torch.float32)):
+        if probe is None and not needs_grad and self._for_cluster(mons):
             fast = self._cluster_solve(eps, src, mons)
         if fast is not None:
             specs, field, dfts = fast
@@ -177,6 +172,27 @@ class FDTDSolver2D:
             cache[key] = make()
         return cache[key]
 
+    def _for_cluster(self, mons) -> bool:
+        """Whether a solve without gradient and probe is one for the cluster kernel.  A
+        step there costs what its busiest warp walks, a row in pieces of 32 columns: us per
+        step on B200, where a launch per step takes 6.2 and a resident step 0.4 - 1: 64^2
+        0.8, 100^2 2.5, 256^2 2.9, 270 x 333 5.2 (22 pieces), 256 x 512 5.8 (16); 460 x 400
+        7.7 (26), 64 x 1024 7.3 (32), 64 x 2100 20.6 (66).  A call costs 80 us less of host
+        time than a resident one: us per call in the cluster / resident, 64^2 (2 pieces) 48
+        steps 228 / 264, 64 steps 253 / 266; 100^2 (4) 32 steps 251 / 280, 48 steps 304 /
+        278; 256^2 (8) 16 steps 205 / 261, 32 steps 268 / 262; 407 x 164 (12) 16 steps 225 /
+        292; 256 x 512 (16) 8 steps 216 / 266, 16 steps 280 / 266; 38 x 1128 (36) 3 steps
+        211 / 291.  (FP32 TE and runs of under 8 steps apart, every grid within 24 pieces
+        has a resident plan.)"""
+        T, te32 = self.n_steps, self.polarization == "TE" and self.dtype == torch.float32
+        if not (T <= 60 or te32) or not isinstance(mons or (), (list, tuple)) or \
+                len(mons or ()) > 1:
+            return False
+        H, W = self.grid_shape
+        rows = -(-H // 16)  # per CTA, 16 warps each
+        pieces = -(-rows // 16) * -(-W // 32)
+        return (te32 and pieces <= 24) or T * (4 + pieces) <= 300
+
     def _cluster_solve(self, eps, src, mons):
         """Gradient-free solve with the whole grid in one thread-block cluster
         (``dn_batch2d_forward_cluster``) when the grid fits and there is at most
@@ -195,17 +211,9 @@ class FDTDSolver2D:
         return specs, fields[0], [d for d in dfts if d is not None]
 
     def _make_cluster(self, src: dict, specs):
-        """The batch of one that ``_cluster_solve`` runs, None when it cannot or would be
-        slower.  A step of the cluster kernel costs what its busiest warp walks, a row in
-        pieces of 32 columns: us per step in the cluster, B200, where a launch per step
-        takes 6.2: 64^2 0.8, 100^2 2.5, 256^2 2.9, 270 x 333 5.2 (22 pieces), 256 x 512
-        5.8 (16); 460 x 400 7.7 (26), 64 x 1024 7.3 (32), 64 x 2100 20.6 (66)."""
+        """The batch of one that ``_cluster_solve`` runs, None when it cannot."""
         from diffnano_b200.solvers.batch2d import BatchInstance, FDTDBatch2D, fits_cluster
 
-        H, W = self.grid_shape
-        rows = -(-H // 16)  # per CTA, 16 warps each
-        if -(-rows // 16) * -(-W // 32) > 24:
-            return None
         mon = None
         if len(specs) > 1 or (specs and specs[0].component !=
                               _lib.COMPONENTS[self._fields()[0]]):

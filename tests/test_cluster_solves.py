@@ -46,9 +46,24 @@ def _forward(monkeypatch, solver, *a, **kw):
         return rec, solver.forward(*a, **kw)
 
 
+@pytest.mark.parametrize("shape,pol,dtype,T,want", [
+    ((100, 100), "TM", F32, 37, True), ((100, 100), "TM", F32, 38, False),
+    ((256, 256), "TM", F64, 25, True), ((256, 256), "TM", F64, 26, False),
+    ((16, 32), "TM", F32, 60, True), ((16, 32), "TM", F32, 61, False),
+    ((256, 768), "TM", F32, 10, True), ((256, 769), "TM", F32, 11, False),
+    ((256, 768), "TE", F32, 500, True), ((257, 513), "TE", F32, 500, False),
+    ((257, 513), "TE", F32, 7, True), ((256, 256), "TE", F64, 500, False)])
+def test_which_solves_are_for_the_cluster(shape, pol, dtype, T, want):
+    s = dn.FDTDSolver2D(grid_shape=shape, polarization=pol, n_steps=T, dtype=dtype)
+    assert s._for_cluster(None) == s._for_cluster([{"row": 3}]) == want
+    assert not s._for_cluster([{"row": 3}, {"row": 4}])
+    assert not s._for_cluster(m for m in [{"row": 3}])  # (not looked into)
+
+
 # (shape, polarisation, type, steps): FP32 TE, a row of 24 pieces, a few steps
 CASES = [((100, 100), "TE", F32, 60), ((131, 77), "TE", F32, 60), ((20, 768), "TE", F32, 60),
-         ((100, 100), "TM", F32, 5), ((100, 100), "TE", F64, 7)]
+         ((100, 100), "TM", F32, 5), ((100, 100), "TE", F64, 7), ((129, 131), "TM", F32, 33), ((129, 131), "TM", F64, 20),
+         ((20, 1128), "TM", F32, 3)]
 
 
 @pytest.mark.gpu
@@ -86,11 +101,11 @@ def test_other_solves_keep_their_path(cuda, monkeypatch):
     for pol, kw, probe in (("TM", {}, None), ("TE", {}, [3, 4]), ("TE", {"monitors": two}, None),
                            ("TE", {"monitors": other}, None), ("TE", {"grid_shape": (20, 769)}, None),
                            ("TM", {"grid_shape": (40, 2100)}, None)):
-        s = dn.FDTDSolver2D(polarization=pol, n_steps=40, device=cuda, **kw)
+        s = dn.FDTDSolver2D(polarization=pol, n_steps=60, device=cuda, **kw)
         e = eps.new_full(s.grid_shape, 2.0)
         rec, r = _forward(monkeypatch, s, e, source={**src, **({"probe": probe} if probe else {})})
         assert rec.ran == [] and len(s._engine_cache) == 1
     e = eps.clone().requires_grad_(True)
-    rec, r = _forward(monkeypatch, dn.FDTDSolver2D(polarization="TE", n_steps=40, device=cuda), e,
+    rec, r = _forward(monkeypatch, dn.FDTDSolver2D(polarization="TE", n_steps=60, device=cuda), e,
                       source=src)
     assert rec.ran == [] and r.field.requires_grad
