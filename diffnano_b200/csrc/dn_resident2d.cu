@@ -64,7 +64,8 @@ Plan2d make_plan2d(const dn_grid* g, const dn_source* src, const dn_monitor* mon
   if (nsteps < MIN_STEPS || (g->pitch_y * elem) % 16 != 0) return P;
   if (src && src->component != DN_NONE && src->component != first) return P;
   // the TE update of these equations grows without bound (FP32 overflows within
-  // ~130 steps): FP32 TE runs are short, and stay launch by launch
+  // ~130 steps): FP32 TE has no resident form (FDTDSolver2D takes dn_batch2d.cu's
+  // cluster kernel for it where that is faster than a launch per step)
   if (g->pol == DN_TE && (adjoint || g->dtype == DN_F32)) return P;
   // what a monitor adds in the reverse sweep goes to lambda_Ez alone
   for (int m = 0; adjoint && m < n_mon; ++m)
